@@ -9,6 +9,7 @@
 
 #include "devbuf.h"
 #include "eltwise.h"
+#include "host_stage.h"
 #include "igemm.h"
 #include "internal.h"
 #include "layout.h"
@@ -45,8 +46,9 @@ struct ResolvedRequant {
   std::vector<int32_t> multiplier, shift;
 };
 
+// `cached` (optional): the arrays d_mult / d_shift hold from an earlier call; equal ones are not uploaded again.
 int make_epilogue(const ResolvedRequant& r, const int32_t* d_bias, DevBuf& d_mult, DevBuf& d_shift, cudaStream_t s,
-                  Epilogue* e) {
+                  Epilogue* e, ResolvedRequant* cached = nullptr) {
   e->dialect = r.dialect;
   e->round_mode = r.round_mode;
   e->per_channel = r.per_channel;
@@ -58,14 +60,19 @@ int make_epilogue(const ResolvedRequant& r, const int32_t* d_bias, DevBuf& d_mul
   e->multiplier = nullptr;
   e->shift = nullptr;
   if (!r.multiplier.empty()) {
-    B200Q_TRY(d_mult.upload(r.multiplier.data(), r.multiplier.size() * 4, s));
+    if (!cached || cached->multiplier != r.multiplier) B200Q_TRY(d_mult.upload(r.multiplier.data(), r.multiplier.size() * 4, s));
     e->multiplier = d_mult.as<int32_t>();
   }
   if (!r.shift.empty()) {
-    B200Q_TRY(d_shift.upload(r.shift.data(), r.shift.size() * 4, s));
+    if (!cached || cached->shift != r.shift) B200Q_TRY(d_shift.upload(r.shift.data(), r.shift.size() * 4, s));
     e->shift = d_shift.as<int32_t>();
   }
+  if (cached) *cached = r;
   return B200Q_OK;
+}
+
+int timeout_error(int status, const char* what) {
+  return set_error(B200Q_ERR_TIMEOUT, "%s: a bounded wait inside the kernel ran out (wait site %d)", what, status);
 }
 
 int read_status(DevBuf& d_status, cudaStream_t s, const char* what) {
@@ -74,7 +81,7 @@ int read_status(DevBuf& d_status, cudaStream_t s, const char* what) {
   CUDA_TRY(cudaStreamSynchronize(s));
   if (h != 0) {
     cudaMemsetAsync(d_status.p, 0, 4, s);
-    return set_error(B200Q_ERR_TIMEOUT, "%s: a bounded wait inside the kernel ran out (wait site %d)", what, h);
+    return timeout_error(h, what);
   }
   return B200Q_OK;
 }
@@ -190,6 +197,8 @@ int gemm_dispatch(const void* a, int a_dt, const void* b_nk, int b_dt, int64_t M
 
 struct MatMulHandle {
   DevBuf stage_f32, a_q8, b_f32, b_nk, bias, mult, shift, out_q, out_f32, status, perm;
+  HostStage host;
+  ResolvedRequant requant;   // what mult / shift hold
   bool weights_ready = false;
   int weight_version = -1;
   const float* weight_ptr = nullptr;
@@ -244,7 +253,8 @@ struct ConvHandle {
   Epilogue epi{};
   DevBuf w_oihw, w_packed, bias, mult, shift, x_bordered, a_cols, status;
   // operator-face staging
-  DevBuf x_f32, x_q8, y_q, y_f32, w_f32, bias_f32;
+  DevBuf w_f32, bias_f32;
+  HostStage host;   // host copies pipelined over pieces of the batch
   // operator face: which host filter the device copy was made from (b200q_conv2d_desc::weight_version)
   int weight_version = -1;
   const float* weight_ptr = nullptr;
@@ -265,24 +275,8 @@ struct ConvHandle {
     ++runs_recorded;
     return B200Q_OK;
   }
-  // operator face: host copies pipelined over pieces of the batch (copy-in, compute, copy-out streams)
-  cudaStream_t pipe[3] = {nullptr, nullptr, nullptr};
-  std::vector<cudaEvent_t> pipe_ev;
-  int ensure_pipe(int pieces) {
-    for (int i = 0; i < 3; ++i)
-      if (!pipe[i]) CUDA_TRY(cudaStreamCreateWithFlags(&pipe[i], cudaStreamNonBlocking));
-    while ((int)pipe_ev.size() < 2 * pieces) {
-      cudaEvent_t e;
-      CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      pipe_ev.push_back(e);
-    }
-    return B200Q_OK;
-  }
   ~ConvHandle() {
     for (auto& e : events) cudaEventDestroy(e);
-    for (auto& e : pipe_ev) cudaEventDestroy(e);
-    for (auto& st : pipe)
-      if (st) cudaStreamDestroy(st);
   }
 };
 
@@ -382,7 +376,7 @@ int conv_setup(ConvHandle* h, const b200q_conv2d_desc& d, const void* w_dev, int
   return B200Q_OK;
 }
 
-// x: device NCHW (bytes, or float holding integers); y: device NCHW native out dtype
+// x: device NCHW bytes; y: device NCHW native out dtype
 // `images` < 0: the whole batch of the descriptor; otherwise the first `images` images of x / y (the operator face
 // pipelines its host copies over pieces of the batch)
 // The transposed product for a channels-last output: the GEMM's rows are the output channels (left operand = the
@@ -426,7 +420,7 @@ void make_transposed(IGemmProblem* p, int oc) {
 // whole 16-byte channel runs)
 // `add`: fuse a tpu.Add of the output with add->residual (same shape and layout as y) into the epilogue; y then
 // receives the Add's result and the convolution's own output is not stored (tensor-core routes only)
-int conv_run(ConvHandle* h, const void* x, int x_is_f32, void* y, cudaStream_t s, long long images = -1, bool x_nhwc = false,
+int conv_run(ConvHandle* h, const void* x, void* y, int* status, cudaStream_t s, long long images = -1, bool x_nhwc = false,
              bool y_nhwc = false, const b200q_fused_add* add = nullptr) {
   auto set_add = [&](IGemmProblem* p) {
     if (!add) return;
@@ -451,7 +445,7 @@ int conv_run(ConvHandle* h, const void* x, int x_is_f32, void* y, cudaStream_t s
   if (nb == 0) return B200Q_OK;
   if ((x_nhwc || y_nhwc) && !(h->use_tc || h->use_im2col))
     return set_error(B200Q_ERR_UNSUPPORTED, "conv2d: channels-last tensors need one of the tensor-core routes");
-  if (x_nhwc && (x_is_f32 || d.ic % 16 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0))
+  if (x_nhwc && (d.ic % 16 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0))
     return set_error(B200Q_ERR_UNSUPPORTED, "conv2d: a channels-last input is 16-byte aligned bytes with channels %% 16 == 0");
   if (h->profiling && (h->use_tc || h->use_im2col)) B200Q_TRY(h->next_triple());
   if (h->use_tc) {
@@ -462,7 +456,7 @@ int conv_run(ConvHandle* h, const void* x, int x_is_f32, void* y, cudaStream_t s
     } else if (x_nhwc) {
       B200Q_TRY(nhwc_to_bordered_launch(x, h->x_bordered.p, nb, (int)d.ic, (int)d.ih, (int)d.iw, h->bh, h->bw, s));
     } else {
-      B200Q_TRY(nchw_to_bordered_nhwc(x, x_is_f32, h->x_bordered.p, (int)nb, (int)d.ic, (int)d.ih, (int)d.iw, h->bh, h->bw, s));
+      B200Q_TRY(nchw_to_bordered_nhwc(x, h->x_bordered.p, (int)nb, (int)d.ic, (int)d.ih, (int)d.iw, h->bh, h->bw, s));
     }
     if (h->profiling) CUDA_TRY(cudaEventRecord(h->ev[1], s));
     IGemmProblem p{};
@@ -503,7 +497,7 @@ int conv_run(ConvHandle* h, const void* x, int x_is_f32, void* y, cudaStream_t s
     if (y_nhwc && d.kh * d.kw == 1 && h->bh == 0 && h->bw == 0 && transposed_product_ok(h->epi, (int)d.oc, p.rows))
       make_transposed(&p, (int)d.oc);
     set_add(&p);
-    B200Q_TRY(igemm_i8_tcgen05_launch(p, h->epi, h->status.as<int>(), s));
+    B200Q_TRY(igemm_i8_tcgen05_launch(p, h->epi, status, s));
     if (h->profiling) CUDA_TRY(cudaEventRecord(h->ev[2], s));
     return B200Q_OK;
   }
@@ -515,15 +509,15 @@ int conv_run(ConvHandle* h, const void* x, int x_is_f32, void* y, cudaStream_t s
                                    (int)d.sh, (int)d.sw, (int)d.dh, (int)d.dw, -(int)d.pht, -(int)d.pwl, h->kpad, s));
     } else if (h->few_channels) {
       // few input channels (a network's stem): rows are built from 8-byte runs of the NCHW input
-      B200Q_TRY(im2col_few_channels_launch(x, x_is_f32, h->a_cols.p, nb, (int)d.ic, (int)d.ih, (int)d.iw, h->g.oh, h->g.ow,
+      B200Q_TRY(im2col_few_channels_launch(x, h->a_cols.p, nb, (int)d.ic, (int)d.ih, (int)d.iw, h->g.oh, h->g.ow,
                                            (int)d.kh, (int)d.sh, (int)d.sw, (int)d.pht, (int)d.pwl, h->kpad, s));
     } else if (d.ic <= 4) {
       // few input channels, other geometry: rows are gathered byte by byte straight from the NCHW input
-      B200Q_TRY(im2col_nchw_small_c_launch(x, x_is_f32, h->a_cols.p, nb, (int)d.ic, (int)d.ih, (int)d.iw, h->g.oh, h->g.ow,
+      B200Q_TRY(im2col_nchw_small_c_launch(x, h->a_cols.p, nb, (int)d.ic, (int)d.ih, (int)d.iw, h->g.oh, h->g.ow,
                                            (int)d.kh, (int)d.kw, (int)d.sh, (int)d.sw, (int)d.dh, (int)d.dw, (int)d.pht,
                                            (int)d.pwl, h->kpad, s));
     } else {
-      B200Q_TRY(nchw_to_bordered_nhwc(x, x_is_f32, h->x_bordered.p, (int)nb, (int)d.ic, (int)d.ih, (int)d.iw, h->bh, h->bw, s));
+      B200Q_TRY(nchw_to_bordered_nhwc(x, h->x_bordered.p, (int)nb, (int)d.ic, (int)d.ih, (int)d.iw, h->bh, h->bw, s));
       B200Q_TRY(im2col_nhwc_launch(h->x_bordered.p, h->a_cols.p, nb, (int)d.ic, h->Hp, h->Wp, h->g.oh, h->g.ow, (int)d.kh,
                                    (int)d.kw, (int)d.sh, (int)d.sw, (int)d.dh, (int)d.dw, h->bh - (int)d.pht,
                                    h->bw - (int)d.pwl, h->kpad, s));
@@ -548,20 +542,13 @@ int conv_run(ConvHandle* h, const void* x, int x_is_f32, void* y, cudaStream_t s
     p.dependent_launch = h->profiling ? 0 : 1;
     if (y_nhwc && transposed_product_ok(h->epi, (int)d.oc, p.rows)) make_transposed(&p, (int)d.oc);
     set_add(&p);
-    B200Q_TRY(igemm_i8_tcgen05_launch(p, h->epi, h->status.as<int>(), s));
+    B200Q_TRY(igemm_i8_tcgen05_launch(p, h->epi, status, s));
     if (h->profiling) CUDA_TRY(cudaEventRecord(h->ev[2], s));
     return B200Q_OK;
   }
-  const void* xin = x;
-  if (x_is_f32) {
-    const long long n = nb * d.ic * d.ih * d.iw;
-    B200Q_TRY(h->x_q8.ensure((size_t)n));
-    B200Q_TRY(f32_to_q8((const float*)x, h->x_q8.p, n, s));
-    xin = h->x_q8.p;
-  }
   ConvGeometry g = h->g;
   g.n = (int)nb;
-  return conv2d_i8_direct_launch(xin, d.input_dtype == B200Q_DT_U8, h->w_oihw.as<int8_t>(), g, h->epi, y, s);
+  return conv2d_i8_direct_launch(x, d.input_dtype == B200Q_DT_U8, h->w_oihw.as<int8_t>(), g, h->epi, y, s);
 }
 
 // tensor_hc_transpose (include/tpu_mlir/Support/MathUtils.h:213-228): src [n][c][h][w] -> dst [n][h][c][w]
@@ -657,9 +644,25 @@ int b200q_matmul_inference(const b200q_matmul_desc* desc, float* const* inputs, 
       h->weight_version = d.weight_version;
       h->weight_ptr = inputs[1];
     }
+    if (a_elems == 0) break;
+    if (!d.right_batched && !d.is_cv18xx && !hdim && !left_t && !out_t) {
+      // one product whose rows are the pieces the host conversions, the link and the kernels overlap on
+      ResolvedRequant r;
+      Epilogue e;
+      if ((rc = resolve_matmul(d, multi_f, 0, &r))) break;
+      if ((rc = make_epilogue(r, bias_f ? h->bias.as<int32_t>() : nullptr, h->mult, h->shift, s, &e, &h->requant))) break;
+      int status = 0;
+      rc = h->host.run(inputs[0], outputs[0], rows, (size_t)d.K, (size_t)d.N, d.out_dtype, dtype_size(d.out_dtype), &status,
+                       [&](int64_t, int64_t cnt, const uint8_t* x, void* y, int* st_dev, cudaStream_t st) {
+                         return gemm_dispatch(x, d.input_dtype, h->b_nk.p, d.right_dtype, cnt, d.N, d.K, d.input_zp, d.right_zp, e, y, st_dev,
+                                              d.algo, st);
+                       });
+      if (rc == B200Q_OK && status != 0) rc = timeout_error(status, "matmul");
+      break;
+    }
     if ((rc = h->status.ensure(4))) break;
     if (cudaMemsetAsync(h->status.p, 0, 4, s) != cudaSuccess) { rc = cuda_error(cudaGetLastError(), "memset", __FILE__, __LINE__); break; }
-    if (a_elems == 0) break;
+    h->requant = ResolvedRequant();   // the arrays below are uploaded once per batch entry
     if ((rc = h->stage_f32.ensure(a_elems * 4 > (size_t)d.N * 4 ? a_elems * 4 : (size_t)d.N * 4))) break;
     if ((rc = h->a_q8.ensure(a_elems))) break;
     if ((rc = h->out_q.ensure(o_elems * dtype_size(d.out_dtype)))) break;
@@ -797,66 +800,14 @@ int b200q_conv2d_inference(const b200q_conv2d_desc* desc, float* const* inputs, 
     B200Q_TRY(conv_upload_weights(h, *desc, inputs, n_inputs, s));
   }
   const b200q_conv2d_desc& d = h->d;
-  const size_t x_elems = (size_t)d.n * d.ic * d.ih * d.iw;
-  const size_t y_elems = (size_t)d.n * d.oc * h->g.oh * h->g.ow;
-  if (x_elems == 0) return B200Q_OK;
-  B200Q_TRY(h->x_f32.ensure(x_elems * 4));
-  B200Q_TRY(h->y_q.ensure(y_elems * dtype_size(d.out_dtype)));
-  B200Q_TRY(h->y_f32.ensure(y_elems * 4));
-  // The float ABI makes this call a PCIe transfer with a convolution in the middle: the batch is cut into pieces so
-  // that the upload of piece i+1, the kernels of piece i and the download of piece i-1 overlap (both directions of
-  // the link at once; the host buffers should be pinned for that).
-  const size_t xi = (size_t)d.ic * d.ih * d.iw, yi = (size_t)d.oc * h->g.oh * h->g.ow;  // elements per image
-  // The first upload and the last download overlap with nothing, which favours many pieces; every piece costs
-  // launches and stream hand-offs, which favours few.  Measured on config 1 (103 MB each way): 8 pieces 2.59 ms,
-  // 16 pieces 2.76 ms, 32 pieces 3.32 ms.  Pieces are >= 2 MB, at most 8 (B200Q_CONV_PIECES overrides the count).
-  static const int max_pieces = [] {
-    const char* v = getenv("B200Q_CONV_PIECES");
-    const int n = v ? atoi(v) : 0;
-    return n >= 1 && n <= 1024 ? n : 8;
-  }();
-  const long long min_imgs = (long long)((((size_t)2 << 20) + xi * 4 - 1) / (xi * 4));
-  const long long even = (d.n + max_pieces - 1) / max_pieces;
-  long long per = even > min_imgs ? even : min_imgs;
-  if (per > d.n) per = d.n;
-  const int pieces = (int)((d.n + per - 1) / per);
-  int rc = B200Q_OK;
-  if (pieces <= 1) {
-    CUDA_TRY(cudaMemcpyAsync(h->x_f32.p, inputs[0], x_elems * 4, cudaMemcpyHostToDevice, s));
-    rc = conv_run(h, h->x_f32.p, 1, h->y_q.p, s);
-    if (rc == B200Q_OK) rc = q_to_f32(h->y_q.p, d.out_dtype, h->y_f32.as<float>(), (long long)y_elems, s);
-    if (rc == B200Q_OK && cudaMemcpyAsync(outputs[0], h->y_f32.p, y_elems * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess)
-      rc = cuda_error(cudaGetLastError(), "D2H output", __FILE__, __LINE__);
-    if (rc == B200Q_OK) rc = read_status(h->status, s, "conv2d");
-    else cudaStreamSynchronize(s);
-    return rc;
-  }
-  CUDA_TRY(cudaStreamSynchronize(s));  // whatever the caller queued on the default stream comes first
-  B200Q_TRY(h->ensure_pipe(pieces));
-  cudaStream_t s_in = h->pipe[0], s_cmp = h->pipe[1], s_out = h->pipe[2];
-  const size_t ysz = dtype_size(d.out_dtype);
-  for (int c = 0; c < pieces && rc == B200Q_OK; ++c) {
-    const long long i0 = (long long)c * per, cnt = (i0 + per <= d.n) ? per : d.n - i0;
-    float* xd = h->x_f32.as<float>() + (size_t)i0 * xi;
-    uint8_t* yq = h->y_q.as<uint8_t>() + (size_t)i0 * yi * ysz;
-    float* yd = h->y_f32.as<float>() + (size_t)i0 * yi;
-    CUDA_TRY(cudaMemcpyAsync(xd, inputs[0] + (size_t)i0 * xi, (size_t)cnt * xi * 4, cudaMemcpyHostToDevice, s_in));
-    CUDA_TRY(cudaEventRecord(h->pipe_ev[2 * c], s_in));
-    CUDA_TRY(cudaStreamWaitEvent(s_cmp, h->pipe_ev[2 * c], 0));
-    rc = conv_run(h, xd, 1, yq, s_cmp, cnt);
-    if (rc == B200Q_OK) rc = q_to_f32(yq, d.out_dtype, yd, (long long)((size_t)cnt * yi), s_cmp);
-    if (rc != B200Q_OK) break;
-    CUDA_TRY(cudaEventRecord(h->pipe_ev[2 * c + 1], s_cmp));
-    CUDA_TRY(cudaStreamWaitEvent(s_out, h->pipe_ev[2 * c + 1], 0));
-    CUDA_TRY(cudaMemcpyAsync(outputs[0] + (size_t)i0 * yi, yd, (size_t)cnt * yi * 4, cudaMemcpyDeviceToHost, s_out));
-  }
-  if (rc == B200Q_OK) {
-    CUDA_TRY(cudaStreamSynchronize(s_out));
-    rc = read_status(h->status, s_cmp, "conv2d");
-  } else {
-    for (auto& st : h->pipe) cudaStreamSynchronize(st);
-  }
-  return rc;
+  if (d.n == 0) return B200Q_OK;
+  // the images are the pieces the host conversions, both directions of the link and the kernels overlap on
+  int status = 0;
+  B200Q_TRY(h->host.run(inputs[0], outputs[0], d.n, (size_t)d.ic * d.ih * d.iw, (size_t)d.oc * h->g.oh * h->g.ow, d.out_dtype,
+                        dtype_size(d.out_dtype), &status, [h](int64_t, int64_t cnt, const uint8_t* x, void* y, int* st_dev, cudaStream_t st) {
+                          return conv_run(h, x, y, st_dev, st, cnt);
+                        }));
+  return status == 0 ? B200Q_OK : timeout_error(status, "conv2d");
 }
 
 int b200q_conv2d_dev_create(const b200q_conv2d_desc* desc, const void* filter_oihw_s8, const int32_t* bias_s32, void** handle) {
@@ -876,14 +827,14 @@ int b200q_conv2d_dev_create(const b200q_conv2d_desc* desc, const void* filter_oi
 
 int b200q_conv2d_dev_run(void* handle, const void* x_nchw, void* y_nchw, void* stream) {
   if (!handle || !x_nchw || !y_nchw) return set_error(B200Q_ERR_INVALID, "conv2d_dev_run: null argument");
-  return conv_run(static_cast<ConvHandle*>(handle), x_nchw, 0, y_nchw, static_cast<cudaStream_t>(stream));
+  return conv_run(static_cast<ConvHandle*>(handle), x_nchw, y_nchw, static_cast<ConvHandle*>(handle)->status.as<int>(), static_cast<cudaStream_t>(stream));
 }
 
 int b200q_conv2d_dev_run_layout(void* handle, const void* x, int32_t x_layout, void* y, int32_t y_layout, void* stream) {
   if (!handle || !x || !y) return set_error(B200Q_ERR_INVALID, "conv2d_dev_run_layout: null argument");
   if ((x_layout != B200Q_LAYOUT_NCHW && x_layout != B200Q_LAYOUT_NHWC) || (y_layout != B200Q_LAYOUT_NCHW && y_layout != B200Q_LAYOUT_NHWC))
     return set_error(B200Q_ERR_INVALID, "conv2d_dev_run_layout: unknown layout");
-  return conv_run(static_cast<ConvHandle*>(handle), x, 0, y, static_cast<cudaStream_t>(stream), -1, x_layout == B200Q_LAYOUT_NHWC,
+  return conv_run(static_cast<ConvHandle*>(handle), x, y, static_cast<ConvHandle*>(handle)->status.as<int>(), static_cast<cudaStream_t>(stream), -1, x_layout == B200Q_LAYOUT_NHWC,
                   y_layout == B200Q_LAYOUT_NHWC);
 }
 
@@ -892,7 +843,7 @@ int b200q_conv2d_dev_run_add(void* handle, const void* x, int32_t x_layout, void
   if (!handle || !x || !y || !add) return set_error(B200Q_ERR_INVALID, "conv2d_dev_run_add: null argument");
   if ((x_layout != B200Q_LAYOUT_NCHW && x_layout != B200Q_LAYOUT_NHWC) || (y_layout != B200Q_LAYOUT_NCHW && y_layout != B200Q_LAYOUT_NHWC))
     return set_error(B200Q_ERR_INVALID, "conv2d_dev_run_add: unknown layout");
-  return conv_run(static_cast<ConvHandle*>(handle), x, 0, y, static_cast<cudaStream_t>(stream), -1, x_layout == B200Q_LAYOUT_NHWC,
+  return conv_run(static_cast<ConvHandle*>(handle), x, y, static_cast<ConvHandle*>(handle)->status.as<int>(), static_cast<cudaStream_t>(stream), -1, x_layout == B200Q_LAYOUT_NHWC,
                   y_layout == B200Q_LAYOUT_NHWC, add);
 }
 

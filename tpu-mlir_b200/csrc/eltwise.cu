@@ -13,16 +13,6 @@
 
 namespace b200q {
 namespace {
-__device__ __forceinline__ uint8_t to_u8(uint8_t v) { return v; }
-__device__ __forceinline__ uint8_t to_u8(float v) { return (uint8_t)(int)v; }  // integral by contract
-
-__device__ __forceinline__ uint32_t ld4_as_bytes(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
-__device__ __forceinline__ uint32_t ld4_as_bytes(const float* p) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  return (uint32_t)((int)v.x & 0xff) | ((uint32_t)((int)v.y & 0xff) << 8) | ((uint32_t)((int)v.z & 0xff) << 16) |
-         ((uint32_t)((int)v.w & 0xff) << 24);
-}
-
 
 __device__ __forceinline__ int32_t ld_q(const void* p, long long i, int dt) {
   switch (dt) {
@@ -320,9 +310,8 @@ __global__ void im2col_nhwc_kernel(const uint8_t* __restrict__ x, uint8_t* __res
 // NHWC copy in between.  A thread assembles one 16-byte piece of a row [kpad] with k = (fy*KW + fx)*C + c from
 // single-byte reads (neighbouring rows share them in L1) and stores it once; positions in the padding and the
 // k >= KH*KW*C tail are zero.  The (c, fy, fx) of every k come from a table in shared memory.
-template <typename T>
 __global__ void __launch_bounds__(256)
-im2col_nchw_small_c_kernel(const T* __restrict__ x, uint8_t* __restrict__ a, int C, int H, int W, int OH, int OW, int KH,
+im2col_nchw_small_c_kernel(const uint8_t* __restrict__ x, uint8_t* __restrict__ a, int C, int H, int W, int OH, int OW, int KH,
                            int KW, int sh, int sw, int dh, int dw, int pht, int pwl, int kpad, long long total_units) {
   extern __shared__ int ktab[];  // per k: c | fy << 8 | fx << 16, or -1 past the filter
   const int kk = KH * KW * C;
@@ -344,7 +333,7 @@ im2col_nchw_small_c_kernel(const T* __restrict__ x, uint8_t* __restrict__ a, int
   const int xo = (int)(row % OW), yo = (int)((row / OW) % OH);
   const long long n = row / ((long long)OW * OH);
   const int y0 = yo * sh - pht, x0 = xo * sw - pwl;
-  const T* xn = x + n * (long long)C * H * W;
+  const uint8_t* xn = x + n * (long long)C * H * W;
   uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int b = 0; b < 16; ++b) {
@@ -352,7 +341,7 @@ im2col_nchw_small_c_kernel(const T* __restrict__ x, uint8_t* __restrict__ a, int
     if (e >= 0) {
       const int c = e & 0xff, iy = y0 + ((e >> 8) & 0xff) * dh, ix = x0 + (e >> 16) * dw;
       if (iy >= 0 && iy < H && ix >= 0 && ix < W)
-        w[b >> 2] |= (uint32_t)to_u8(xn[((long long)c * H + iy) * W + ix]) << (8 * (b & 3));
+        w[b >> 2] |= (uint32_t)xn[((long long)c * H + iy) * W + ix] << (8 * (b & 3));
     }
   }
   reinterpret_cast<uint4*>(a + row * kpad)[piece] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -363,9 +352,8 @@ im2col_nchw_small_c_kernel(const T* __restrict__ x, uint8_t* __restrict__ a, int
 // single bytes.  A block stages the input rows of a band of output rows in shared memory (zero padding included),
 // then every thread assembles 16-byte pieces (two segments) with three aligned word reads and two funnel shifts per
 // segment.  The eighth byte of a segment is whatever pixel follows; its filter weight is zero.
-template <typename T>
 __global__ void __launch_bounds__(256)
-im2col_few_channels_kernel(const T* __restrict__ x, uint8_t* __restrict__ a, int C, int H, int W, int OH, int OW, int KH,
+im2col_few_channels_kernel(const uint8_t* __restrict__ x, uint8_t* __restrict__ a, int C, int H, int W, int OH, int OW, int KH,
                            int sh, int sw, int pht, int pwl, int kpad, int band, int wpad, int pwl_s) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // a dependent convolution may set itself up meanwhile
   extern __shared__ __align__(16) uint8_t tile[];  // [C][rows_in][wpad]
@@ -377,7 +365,7 @@ im2col_few_channels_kernel(const T* __restrict__ x, uint8_t* __restrict__ a, int
   const int tile_words = C * rows_in * wpad / 4;
   for (int i = threadIdx.x; i < tile_words; i += 256) reinterpret_cast<uint32_t*>(tile)[i] = 0u;
   __syncthreads();
-  const T* xn = x + (long long)n * C * H * W;
+  const uint8_t* xn = x + (long long)n * C * H * W;
   if ((W & 3) == 0) {
     const int wq = W / 4;
     for (int i = threadIdx.x; i < C * rows_in * wq; i += 256) {
@@ -385,14 +373,14 @@ im2col_few_channels_kernel(const T* __restrict__ x, uint8_t* __restrict__ a, int
       const int r = cr % rows_in, c = cr / rows_in;
       const int iy = iy0 + r;
       if (iy >= 0 && iy < H)
-        *reinterpret_cast<uint32_t*>(tile + (c * rows_in + r) * wpad + pwl_s + 4 * q) = ld4_as_bytes(xn + ((long long)c * H + iy) * W + 4 * q);
+        *reinterpret_cast<uint32_t*>(tile + (c * rows_in + r) * wpad + pwl_s + 4 * q) = *reinterpret_cast<const uint32_t*>(xn + ((long long)c * H + iy) * W + 4 * q);
     }
   } else {
     for (int i = threadIdx.x; i < C * rows_in * W; i += 256) {
       const int q = i % W, cr = i / W;
       const int r = cr % rows_in, c = cr / rows_in;
       const int iy = iy0 + r;
-      if (iy >= 0 && iy < H) tile[(c * rows_in + r) * wpad + pwl_s + q] = to_u8(xn[((long long)c * H + iy) * W + q]);
+      if (iy >= 0 && iy < H) tile[(c * rows_in + r) * wpad + pwl_s + q] = xn[((long long)c * H + iy) * W + q];
     }
   }
   __syncthreads();
@@ -719,7 +707,7 @@ int im2col_nhwc_launch(const void* x, void* a, long long N, int C, int Hp, int W
   return B200Q_OK;
 }
 
-int im2col_nchw_small_c_launch(const void* x, int x_is_f32, void* a, long long N, int C, int H, int W, int OH, int OW, int KH,
+int im2col_nchw_small_c_launch(const void* x, void* a, long long N, int C, int H, int W, int OH, int OW, int KH,
                                int KW, int sh, int sw, int dh, int dw, int pht, int pwl, int kpad, cudaStream_t s) {
   if (kpad % 16 != 0 || (reinterpret_cast<uintptr_t>(a) & 15) != 0 || KH > 255 || KW > 255 || C > 255)
     return set_error(B200Q_ERR_INVALID, "im2col (small C): row length and buffer must be 16-byte aligned");
@@ -727,12 +715,8 @@ int im2col_nchw_small_c_launch(const void* x, int x_is_f32, void* a, long long N
   if (units == 0) return B200Q_OK;
   if ((units + 255) / 256 > 0x7fffffffLL) return set_error(B200Q_ERR_UNSUPPORTED, "im2col: too large");
   const size_t smem = (size_t)kpad * sizeof(int);
-  if (x_is_f32)
-    im2col_nchw_small_c_kernel<float><<<nblk(units, 256), 256, smem, s>>>((const float*)x, (uint8_t*)a, C, H, W, OH, OW, KH, KW,
-                                                                            sh, sw, dh, dw, pht, pwl, kpad, units);
-  else
-    im2col_nchw_small_c_kernel<uint8_t><<<nblk(units, 256), 256, smem, s>>>((const uint8_t*)x, (uint8_t*)a, C, H, W, OH, OW, KH,
-                                                                              KW, sh, sw, dh, dw, pht, pwl, kpad, units);
+  im2col_nchw_small_c_kernel<<<nblk(units, 256), 256, smem, s>>>((const uint8_t*)x, (uint8_t*)a, C, H, W, OH, OW, KH, KW, sh, sw, dh, dw,
+                                                                 pht, pwl, kpad, units);
   CUDA_TRY(cudaGetLastError());
   return B200Q_OK;
 }
@@ -746,7 +730,7 @@ bool im2col_few_channels_ok(int C, int H, int W, int KH, int KW, int sh, int sw,
   return (size_t)C * rows_in * wpad <= 96 * 1024;
 }
 
-int im2col_few_channels_launch(const void* x, int x_is_f32, void* a, long long N, int C, int H, int W, int OH, int OW, int KH,
+int im2col_few_channels_launch(const void* x, void* a, long long N, int C, int H, int W, int OH, int OW, int KH,
                                int sh, int sw, int pht, int pwl, int kpad, cudaStream_t s) {
   if (N == 0) return B200Q_OK;
   if (N > 65535) return set_error(B200Q_ERR_UNSUPPORTED, "im2col (few channels): at most 65535 images per call");
@@ -757,15 +741,9 @@ int im2col_few_channels_launch(const void* x, int x_is_f32, void* a, long long N
   const int wpad = ((max((OW - 1) * sw - pwl + pwl_s + 8, pwl_s + W) + 3) & ~3) + 4;  // + one word: the third read of a window
   const size_t smem = (size_t)C * ((band - 1) * sh + KH) * wpad;
   dim3 grid((OH + band - 1) / band, (unsigned)N);
-  if (x_is_f32) {
-    auto k = im2col_few_channels_kernel<float>;
-    if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, 256, smem, s>>>((const float*)x, (uint8_t*)a, C, H, W, OH, OW, KH, sh, sw, pht, pwl, kpad, band, wpad, pwl_s);
-  } else {
-    auto k = im2col_few_channels_kernel<uint8_t>;
-    if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<grid, 256, smem, s>>>((const uint8_t*)x, (uint8_t*)a, C, H, W, OH, OW, KH, sh, sw, pht, pwl, kpad, band, wpad, pwl_s);
-  }
+  if (smem > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(im2col_few_channels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  im2col_few_channels_kernel<<<grid, 256, smem, s>>>((const uint8_t*)x, (uint8_t*)a, C, H, W, OH, OW, KH, sh, sw, pht, pwl, kpad, band,
+                                                     wpad, pwl_s);
   CUDA_TRY(cudaGetLastError());
   return B200Q_OK;
 }

@@ -5,8 +5,8 @@
 
 namespace b200q {
 
-// x NCHW (uint8/int8 bytes, or float holding integers) -> y [N][H+2bh][W+2bw][C] bytes, interior only.
-int nchw_to_bordered_nhwc(const void* x, int x_is_f32, void* y, int N, int C, int H, int W, int bh, int bw,
+// x NCHW bytes -> y [N][H+2bh][W+2bw][C] bytes, interior only.
+int nchw_to_bordered_nhwc(const void* x, void* y, int N, int C, int H, int W, int bh, int bw,
                           cudaStream_t s);
 // w [OC][IC][KH][KW] -> [OC][KH*KW][IC] bytes.
 int repack_weight_oihw(const void* w, int w_is_f32, void* wr, int OC, int IC, int KH, int KW, cudaStream_t s);
