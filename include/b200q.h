@@ -449,6 +449,30 @@ int b200q_calib_minmax_noalloc(const float *x, int64_t n_per_sample, int64_t sam
 int b200q_calib_histogram(void *ctx, const float *x, int64_t n_per_sample, int64_t samples, const float *th_host,
                           const int32_t *nbins_host, int32_t *hist, int64_t hist_len, void *stream);
 
+/* The two statistics over many tensors of one batch of samples (a network's activations) with one launch each: tensor t
+ * is x[t][samples][n_per_sample[t]] on the device.  minmax_host [tensors][samples][2] is filled on return (synchronous);
+ * th_host / nbins_host [tensors][samples] and hist[t] / hist_len[t] mean what they mean in b200q_calib_histogram. */
+int b200q_calib_minmax_many(void *ctx, int32_t tensors, const float *const *x, const int64_t *n_per_sample, int64_t samples,
+                            float *minmax_host, void *stream);
+int b200q_calib_histogram_many(void *ctx, int32_t tensors, const float *const *x, const int64_t *n_per_sample, int64_t samples,
+                               const float *th_host, const int32_t *nbins_host, int32_t *const *hist, const int64_t *hist_len,
+                               void *stream);
+
+/* process_statistic + combine_histogram's bookkeeping (kld_calibrator.py:391-398,:462-476; cali_math.py:82-103) of `tensors`
+ * tensors, advanced by `samples` samples whose minmax [tensors][samples][2] are given, in the reference's float32
+ * arithmetic: (threshold, bins) of every sample, 0 where it contributes nothing.  A growth past max_bins starts over with
+ * the sample it happens at (last_reset, counted from first_sample): what was histogrammed for earlier samples is to be
+ * dropped.  Host code, no device needed.  A state starts as {+inf, -inf, 0, 0, 0, 0, 0}. */
+typedef struct {
+  float min, max;      /* running extrema */
+  float th, width;     /* threshold of the current histogram and its bin width */
+  int64_t bins;        /* its bins */
+  int64_t last_reset;  /* sample at which it last started over */
+  int64_t started;
+} b200q_bin_state;
+int b200q_calib_bin_schedule(b200q_bin_state *state, int32_t tensors, int64_t samples, const float *minmax, int64_t first_sample,
+                             int32_t bin_num, int64_t max_bins, float *th, int32_t *nbins);
+
 /* Counter layout of the histogram kernel, process-wide: -1 = chosen per launch from the bin count and the work
  * per block (default); 0..4 = 2^mode 32-bit copies of every bin per block; 5 = one 16-bit counter per (bin, lane).
  * Every layout produces the same counts; this only exists to measure them against each other.  (No counterpart in

@@ -186,6 +186,11 @@ SIGNATURES = {
     "b200q_calib_minmax_noalloc": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
     "b200q_calib_histogram": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.POINTER(C.c_float),
                                         C.POINTER(C.c_int32), C.c_void_p, C.c_int64, C.c_void_p]),
+    "b200q_calib_minmax_many": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]),
+    "b200q_calib_histogram_many": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
+                                             C.c_void_p, C.c_void_p]),
+    "b200q_calib_bin_schedule": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64, C.c_void_p, C.c_int64, C.c_int32, C.c_int64, C.c_void_p,
+                                           C.c_void_p]),
     "b200q_calib_set_histogram_layout": (None, [C.c_int32]),
     "b200q_calib_find_thresholds": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_void_p), C.POINTER(C.c_int64),
                                               C.POINTER(C.c_float), C.c_int64, C.POINTER(C.c_float),

@@ -98,6 +98,74 @@ minmax_kernel(const float* __restrict__ x, long long n, float* __restrict__ out,
   }
 }
 
+// Many tensors in one launch.  The rows (tensor, sample) are cut into chunks of MANY_CHUNK floats, one block each, so that
+// a launch over a network's activations is one wave after another of equal blocks instead of a kernel (and its tail) per
+// tensor.  A block's extrema meet in two atomics on an order-preserving integer image of the floats; the host maps them
+// back.  73 activations of 16 ResNet-50 samples (711 MB): one launch instead of 73.
+constexpr int MANY_CHUNK = 32768;
+
+__device__ __forceinline__ uint32_t ordered_bits(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
+// the last tensor whose first chunk / element is <= pos
+__device__ __forceinline__ int find_tensor(const CalibTensor* __restrict__ tab, int tensors, long long pos, bool by_chunk) {
+  int lo = 0, hi = tensors - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if ((by_chunk ? tab[mid].first_chunk : tab[mid].first) <= pos) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(MM_THREADS)
+minmax_many_kernel(const CalibTensor* __restrict__ tab, int tensors, int samples, uint32_t* __restrict__ out_min, uint32_t* __restrict__ out_max) {
+  const int t = find_tensor(tab, tensors, blockIdx.x, true);
+  const long long n = tab[t].n;
+  const int per_row = (int)((n + MANY_CHUNK - 1) / MANY_CHUNK);
+  const int c = (int)(blockIdx.x - tab[t].first_chunk);
+  const int s = c / per_row, part = c - s * per_row;
+  const float* p = tab[t].x + (long long)s * n + (long long)part * MANY_CHUNK;
+  const int len = (int)min((long long)MANY_CHUNK, n - (long long)part * MANY_CHUNK);
+  float lo = INFINITY, hi = -INFINITY;
+  int head = (int)(((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) >> 2);
+  if (head > len) head = len;
+  if ((int)threadIdx.x < head) lo = hi = p[threadIdx.x];
+  const int body4 = (len - head) >> 2;
+  const float4* p4 = reinterpret_cast<const float4*>(p + head);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < body4; i += MM_THREADS) {
+    const float4 v = p4[i];
+    lo = fminf(fminf(lo, v.x), fminf(v.y, fminf(v.z, v.w)));
+    hi = fmaxf(fmaxf(hi, v.x), fmaxf(v.y, fmaxf(v.z, v.w)));
+  }
+  const int done = head + body4 * 4;
+  if (done + (int)threadIdx.x < len) {
+    lo = fminf(lo, p[done + threadIdx.x]);
+    hi = fmaxf(hi, p[done + threadIdx.x]);
+  }
+  __shared__ float slo[MM_THREADS / 32], shi[MM_THREADS / 32];
+  lo = warp_min(lo);
+  hi = warp_max(hi);
+  if ((threadIdx.x & 31) == 0) {
+    slo[threadIdx.x >> 5] = lo;
+    shi[threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < MM_THREADS / 32; ++w) {
+      lo = fminf(lo, slo[w]);
+      hi = fmaxf(hi, shi[w]);
+    }
+    if (!(lo != lo)) {   // (a chunk of NaNs alone leaves +-infinity, which changes nothing)
+      atomicMin(&out_min[(long long)t * samples + s], ordered_bits(lo));
+      atomicMax(&out_max[(long long)t * samples + s], ordered_bits(hi));
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------- histogram
 constexpr int HIST_THREADS = 1024;
 constexpr int HIST_SMEM_BYTES = 208 * 1024;        // counters of one block (one block per SM)
@@ -129,17 +197,17 @@ struct HistGeom {
   int cap_words;   // shared-memory words available
 };
 
-// Persistent: block b owns the flat element range [b * piece, (b + 1) * piece) of x[samples][n].  Sample s is
-// histogrammed with its own (threshold th[s], bins nb[s]) and ADDED into the first nb[s] entries of hist; nb[s] == 0
-// skips the sample.  Counters stay in shared memory across samples that share (threshold, bins) and are merged into
-// hist when the geometry changes, before a 16-bit counter could overflow, and at the end.
+// Persistent: the tensors x_t[samples][n_t] of the table lie one behind the other in one flat element order, of which
+// block b owns the range [b * piece, (b + 1) * piece).  Sample s of tensor t is histogrammed with its own (threshold
+// th[t][s], bins nb[t][s]) and ADDED into the first nb[t][s] entries of the tensor's hist; nb == 0 skips the sample.
+// Counters stay in shared memory across samples that share tensor, threshold and bins and are merged into hist when one
+// of them changes, before a 16-bit counter could overflow, and at the end.
 template <bool LANE16>
 __global__ void __launch_bounds__(HIST_THREADS, 1)
-histogram_kernel(const float* __restrict__ x, long long n, long long samples, long long piece, const float* __restrict__ th,
-                 const int* __restrict__ nbv, int* __restrict__ hist, int copies_log2, int cap_words, int zero_words) {
+histogram_kernel(const CalibTensor* __restrict__ tab, int tensors, int samples, long long total, long long piece,
+                 const float* __restrict__ th_all, const int* __restrict__ nb_all, int copies_log2, int cap_words, int zero_words) {
   extern __shared__ unsigned int sh[];
   const int tid = threadIdx.x, lane = tid & 31;
-  const long long total = samples * n;
   const long long begin = (long long)blockIdx.x * piece;
   const long long end = begin + piece < total ? begin + piece : total;
   if (begin >= end) return;
@@ -147,6 +215,7 @@ histogram_kernel(const float* __restrict__ x, long long n, long long samples, lo
   __syncthreads();
 
   int cur_bins = 0;            // geometry of the counters now in shared memory (0: none)
+  int* hist = nullptr;         // where they belong
   uint32_t cur_th = 0;
   bool cur_shared = false;
   long long since_merge = 0;
@@ -190,17 +259,22 @@ histogram_kernel(const float* __restrict__ x, long long n, long long samples, lo
   };
 
   long long pos = begin;
+  int t = find_tensor(tab, tensors, begin, false);
   while (pos < end) {
-    const long long s = pos / n;
-    long long seg_end = (s + 1) * n < end ? (s + 1) * n : end;
-    const int bins = nbv[s];
+    while (t + 1 < tensors && pos >= tab[t + 1].first) ++t;
+    const long long n = tab[t].n, first = tab[t].first;
+    const float* const x = tab[t].x - first;   // indexed by flat position
+    const long long s = (pos - first) / n;
+    long long seg_end = first + (s + 1) * n < end ? first + (s + 1) * n : end;
+    const int bins = nb_all[(long long)t * samples + s];
     if (bins <= 0) {
       pos = seg_end;
       continue;
     }
-    const float thv = th[s];
-    if (bins != cur_bins || __float_as_uint(thv) != cur_th) {
+    const float thv = th_all[(long long)t * samples + s];
+    if (bins != cur_bins || __float_as_uint(thv) != cur_th || tab[t].hist != hist) {
       merge();
+      hist = tab[t].hist;
       cur_bins = bins;
       cur_th = __float_as_uint(thv);
       cur_shared = LANE16 ? (((bins + 1) >> 1) * 32 <= cap_words) : (((long long)bins << copies_log2) <= cap_words);
@@ -325,63 +399,111 @@ __global__ void fold_kernel(const int* __restrict__ in, long long n_in, int* __r
 }
 
 // ------------------------------------------------------------------------------------------- KLD
-// One block per histogram, one thread per candidate threshold i = (m+1)*BINS.  Every float sum runs in the
-// reference's order (sequential, left to right) because the counts exceed 2^24 and float addition is not
-// associative; the log10 terms are formed in double and folded into a float accumulator like the reference.
-__global__ void __launch_bounds__(1024)
-kld_kernel(const int* __restrict__ hist_all, const long long* __restrict__ offsets, const float* __restrict__ widths,
-           int BINS, float* __restrict__ thresholds, float* __restrict__ kl_all) {
+// One warp per candidate threshold i = (m+1)*BINS.  Every float sum runs in the reference's order (sequential, left to
+// right) because the counts exceed 2^24 and float addition is not associative; the log10 terms are formed in double and
+// folded into a float accumulator like the reference.  What can be done in any order is spread over the lanes: the two
+// long sums run side by side on two lanes, the bins' sums and logarithms on 32, and of the divergence itself only the
+// chain acc = (float)(acc + term) is serial (one conversion, one double addition and one conversion per non-empty bin).
+// 73 histograms of 2048 to 3000 bins: 1690 us with one thread per candidate, dominated by two log10 calls per bin in a
+// row; see the call's time in the notes of the calibration driver.
+constexpr int KLD_WARPS = 16;
+constexpr int KLD_SMEM_BINS = 40 * 1024;   // histograms up to this length are read from shared memory
+
+struct KldWarp {
+  double qlog[128];
+};
+
+__global__ void __launch_bounds__(KLD_WARPS * 32)
+kld_kernel(const KldTensor* __restrict__ tab, int BINS, float* __restrict__ kl_all, int smem_bins) {
+  extern __shared__ __align__(16) uint8_t kld_smem[];
+  KldWarp* const per_warp = reinterpret_cast<KldWarp*>(kld_smem);
+  int* const sh = reinterpret_cast<int*>(kld_smem + KLD_WARPS * sizeof(KldWarp));
   const int t = blockIdx.x;
-  const int* hist = hist_all + offsets[t];
-  const long long N = offsets[t + 1] - offsets[t];
-  const int KL_NUM = (int)(N / BINS);
-  __shared__ long long scount[32];
-  __shared__ float skl[1024];
-  // total count (exact, int64)
-  long long c = 0;
-  for (long long j = threadIdx.x; j < N; j += blockDim.x) c += hist[j];
+  const int N = tab[t].len, n_in = tab[t].n_in;
+  const int* __restrict__ gh = tab[t].hist;
+  const int KL_NUM = N / BINS;
+  if ((int)blockIdx.y * KLD_WARPS >= KL_NUM) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool in_smem = N <= smem_bins;
+  __shared__ long long scount[KLD_WARPS];
+  long long c = 0;   // total count (exact, int64)
+  for (int j = threadIdx.x; j < N; j += KLD_WARPS * 32) {
+    const int h = j < n_in ? gh[j] : 0;
+    if (in_smem) sh[j] = h;
+    c += h;
+  }
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) scount[threadIdx.x >> 5] = c;
+  if (lane == 0) scount[warp] = c;
   __syncthreads();
   long long count = 0;
-  for (int w = 0; w < (blockDim.x + 31) / 32; ++w) count += scount[w];
+  for (int w = 0; w < KLD_WARPS; ++w) count += scount[w];
   const float fcount = (float)count;
+  auto H = [&](int j) { return in_smem ? sh[j] : (j < n_in ? __ldg(gh + j) : 0); };
 
-  const int m = threadIdx.x;
-  if (m < KL_NUM) {
-    const long long i = (long long)(m + 1) * BINS;
-    float tail = 0.f;  // P[i-1]: hist[i-1 .. N-1] summed left to right
-    for (long long j = i - 1; j < N; ++j) tail = __fadd_rn(tail, (float)hist[j]);
-    float sum = 0.f;
-    for (long long j = 0; j < i; ++j) sum = __fadd_rn(sum, (float)hist[j]);
-    const long long expand = i / BINS;
-    float acc = 0.f;
-    long long idx = 0;
-    for (int b = 0; b < BINS; ++b) {
-      float sum_bin = 0.f, positive = 0.f;
-      for (long long k = 0; k < expand; ++k) {
-        const int h = hist[idx + k];
-        sum_bin = __fadd_rn(sum_bin, (float)h);
-        positive = __fadd_rn(positive, h > 0 ? 1.f : 0.f);
-      }
-      if (positive == 0.f) positive = 1.f;
-      const float q_base = __fdiv_rn(__fdiv_rn(sum_bin, positive), sum);
-      for (long long k = 0; k < expand; ++k, ++idx) {
-        const int h = hist[idx];
-        const float p = __fdiv_rn(idx == i - 1 ? tail : (float)h, fcount);
-        if (p == 0.f) continue;  // the term is exactly +-0 and leaves the accumulator unchanged
-        const float q = h ? q_base : 0.f;
-        const double term = __dmul_rn((double)p, __dsub_rn(log10(__dadd_rn((double)p, 1e-30)),
-                                                           log10(__dadd_rn((double)q, 1e-30))));
-        acc = (float)__dadd_rn((double)acc, term);
+  const int m = (int)blockIdx.y * KLD_WARPS + warp;
+  if (m >= KL_NUM) return;
+  const int expand = m + 1, i = expand * BINS;
+  // lane 0: P's sum, hist[0 .. i-1]; lane 1: P[i-1], hist[i-1 .. N-1]; both left to right
+  float chain = 0.f;
+  {
+    const int from = lane == 0 ? 0 : i - 1, to = lane == 0 ? i : (lane == 1 ? N : 0);
+    int j = from;
+    for (; j + 8 <= to; j += 8) {
+      int v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = H(j + k);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) chain = __fadd_rn(chain, (float)v[k]);
+    }
+    for (; j < to; ++j) chain = __fadd_rn(chain, (float)H(j));
+  }
+  const float sum = __shfl_sync(0xffffffffu, chain, 0), tail = __shfl_sync(0xffffffffu, chain, 1);
+  double* const qlog = per_warp[warp].qlog;
+  for (int b = lane; b < BINS; b += 32) {
+    float sum_bin = 0.f;
+    int positive = 0;
+    for (int k = 0; k < expand; ++k) {
+      const int h = H(b * expand + k);
+      sum_bin = __fadd_rn(sum_bin, (float)h);
+      positive += h > 0;
+    }
+    const float q = __fdiv_rn(__fdiv_rn(sum_bin, positive ? (float)positive : 1.f), sum);
+    qlog[b] = log10(__dadd_rn((double)q, 1e-30));
+  }
+  __syncwarp();
+  const double qlog0 = log10(__dadd_rn(0.0, 1e-30));
+  float acc = 0.f;
+  for (int base = 0; base < i; base += 32) {   // BINS is a multiple of 8: i need not be one of 32
+    const int idx = base + lane;
+    const int h = idx < i ? H(idx) : 0;
+    const float p = idx < i ? __fdiv_rn(idx == i - 1 ? tail : (float)h, fcount) : 0.f;
+    double term = 0.0;
+    if (p != 0.f)
+      term = __dmul_rn((double)p, __dsub_rn(log10(__dadd_rn((double)p, 1e-30)), h ? qlog[idx / expand] : qlog0));
+    // p == 0: the term is exactly +-0 and leaves the accumulator unchanged
+    unsigned live = __ballot_sync(0xffffffffu, p != 0.f);
+    if (live == 0xffffffffu) {
+#pragma unroll
+      for (int k = 0; k < 32; ++k) acc = (float)__dadd_rn((double)acc, __shfl_sync(0xffffffffu, term, k));
+    } else {
+      while (live) {
+        const int k = __ffs((int)live) - 1;
+        live &= live - 1;
+        acc = (float)__dadd_rn((double)acc, __shfl_sync(0xffffffffu, term, k));
       }
     }
-    skl[m] = acc;
-    if (kl_all) kl_all[(long long)t * 1024 + m] = acc;
   }
+  if (lane == 0) kl_all[(long long)t * 1024 + m] = acc;
+}
+
+// the_min_index (calibration_math.cpp:71-83): first strict minimum
+__global__ void __launch_bounds__(128)
+kld_argmin_kernel(const KldTensor* __restrict__ tab, int BINS, const float* __restrict__ kl_all, float* __restrict__ thresholds) {
+  __shared__ float skl[1024];
+  const int t = blockIdx.x, KL_NUM = tab[t].len / BINS;
+  for (int k = threadIdx.x; k < KL_NUM; k += 128) skl[k] = kl_all[(long long)t * 1024 + k];
   __syncthreads();
   if (threadIdx.x == 0) {
-    // the_min_index (calibration_math.cpp:71-83): first strict minimum
     float best = skl[0];
     int best_m = 0;
     for (int k = 1; k < KL_NUM; ++k)
@@ -389,7 +511,7 @@ kld_kernel(const int* __restrict__ hist_all, const long long* __restrict__ offse
         best = skl[k];
         best_m = k;
       }
-    thresholds[t] = __fmul_rn(__fmul_rn(widths[t], (float)(best_m + 1)), (float)BINS);
+    thresholds[t] = __fmul_rn(__fmul_rn(tab[t].width, (float)(best_m + 1)), (float)BINS);
   }
 }
 
@@ -476,13 +598,12 @@ int minmax_static_launch(const float* x, long long n, long long samples, float* 
 static int g_hist_mode = -1;  // -1: chosen per launch; 0..4: 2^mode copies; 5: lane-owned 16-bit counters
 void histogram_set_mode(int mode) { g_hist_mode = (mode >= 0 && mode <= 5) ? mode : -1; }
 
-int histogram_launch(const float* x, long long n, long long samples, const float* th, const int* nb, int* hist,
+int histogram_launch(const CalibTensor* tab_dev, int tensors, long long samples, long long total, const float* th, const int* nb,
                      int max_bins, cudaStream_t s) {
-  if (samples == 0 || n == 0) return B200Q_OK;
+  if (samples == 0 || total == 0) return B200Q_OK;
   int dev = 0, sms = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const long long total = samples * n;
   // one block per SM; a block's piece is a multiple of one float4 per thread and at least 16 of them
   const long long quantum = 4LL * HIST_THREADS;
   long long blocks = (total + 16 * quantum - 1) / (16 * quantum);
@@ -497,7 +618,8 @@ int histogram_launch(const float* x, long long n, long long samples, const float
   // 42.2 us, sixteen 43.7 us, lane-owned 16-bit counters 46.3 us (two more instructions per element cost more than the
   // conflicts they avoid); on 64 x 100 352 values four copies are the fastest (20.0 us).  Copies also keep skewed data
   // (everything in a few bins) from serialising on one address.  Fewer copies when the bins do not fit, or when a
-  // block would spend more than a quarter of its element count clearing and summing counters.
+  // block would spend more than a quarter of its element count clearing and summing counters.  (max_bins is the largest
+  // bin count of the call that fits at all; a sample with more bins than that counts straight into global memory.)
   int mode = g_hist_mode;
   if (mode < 0) {
     mode = 2;
@@ -510,8 +632,22 @@ int histogram_launch(const float* x, long long n, long long samples, const float
   const size_t smem = (size_t)(zero_words > 0 ? zero_words : 1) * 4;
   auto kfn = mode == 5 ? histogram_kernel<true> : histogram_kernel<false>;
   CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, HIST_SMEM_BYTES));
-  kfn<<<(unsigned)blocks, HIST_THREADS, smem, s>>>(x, n, samples, piece, th, nb, hist, mode == 5 ? 0 : mode,
+  kfn<<<(unsigned)blocks, HIST_THREADS, smem, s>>>(tab_dev, tensors, (int)samples, total, piece, th, nb, mode == 5 ? 0 : mode,
                                                    (int)zero_words, (int)zero_words);
+  CUDA_TRY(cudaGetLastError());
+  return B200Q_OK;
+}
+
+int histogram_max_shared_bins() { return HIST_SMEM_BYTES / 4; }
+
+long long minmax_many_chunks(long long n, long long samples) { return (n + MANY_CHUNK - 1) / MANY_CHUNK * samples; }
+
+// out_min must hold all ones and out_max zeros; see minmax_many_kernel
+int minmax_many_launch(const CalibTensor* tab_dev, int tensors, long long samples, long long chunks, uint32_t* out_min, uint32_t* out_max,
+                       cudaStream_t s) {
+  if (chunks == 0) return B200Q_OK;
+  if (chunks > 0x7fffffffLL) return set_error(B200Q_ERR_UNSUPPORTED, "minmax: too many elements for one call");
+  minmax_many_kernel<<<(unsigned)chunks, MM_THREADS, 0, s>>>(tab_dev, tensors, (int)samples, out_min, out_max);
   CUDA_TRY(cudaGetLastError());
   return B200Q_OK;
 }
@@ -532,14 +668,17 @@ int fold_launch(const int* in, long long n_in, int* out, long long n_out, cudaSt
   return B200Q_OK;
 }
 
-int kld_launch(const int* hist_all, const long long* offsets_dev, const float* widths_dev, int tensors, int dst_bins,
-               long long max_bins, float* thresholds_dev, float* kl_dev, cudaStream_t s) {
+int kld_launch(const KldTensor* tab_dev, int tensors, int dst_bins, long long max_len, float* thresholds_dev, float* kl_dev, cudaStream_t s) {
   if (tensors == 0) return B200Q_OK;
-  if (dst_bins < 1 || max_bins / dst_bins > 1024)
+  if (dst_bins < 1 || dst_bins > 128 || max_len / dst_bins > 1024)
     return set_error(B200Q_ERR_UNSUPPORTED, "kld: more than 1024 candidates (fold the histogram to at most %d bins first)", 1024 * dst_bins);
-  int threads = (int)((max_bins / dst_bins + 31) / 32 * 32);
-  if (threads < 32) threads = 32;
-  kld_kernel<<<tensors, threads, 0, s>>>(hist_all, offsets_dev, widths_dev, dst_bins, thresholds_dev, kl_dev);
+  const int smem_bins = max_len < KLD_SMEM_BINS ? (int)max_len : KLD_SMEM_BINS;
+  const size_t smem = KLD_WARPS * sizeof(KldWarp) + (size_t)smem_bins * 4;
+  CUDA_TRY(cudaFuncSetAttribute(kld_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(KLD_WARPS * sizeof(KldWarp) + KLD_SMEM_BINS * 4)));
+  const dim3 grid((unsigned)tensors, (unsigned)((max_len / dst_bins + KLD_WARPS - 1) / KLD_WARPS));
+  kld_kernel<<<grid, KLD_WARPS * 32, smem, s>>>(tab_dev, dst_bins, kl_dev, smem_bins);
+  CUDA_TRY(cudaGetLastError());
+  kld_argmin_kernel<<<tensors, 128, 0, s>>>(tab_dev, dst_bins, kl_dev, thresholds_dev);
   CUDA_TRY(cudaGetLastError());
   return B200Q_OK;
 }

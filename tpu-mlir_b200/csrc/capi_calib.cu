@@ -17,7 +17,7 @@ namespace {
 constexpr long long MAX_KLD_BINS = 64 * 2048;  // kld_calibrator.py:338
 
 struct CalibCtx {
-  DevBuf mm_scratch, params, work, work2, offsets, widths, thresholds, kl, stage, mm_out;
+  DevBuf mm_scratch, params, work, work2, table, thresholds, kl, stage, mm_out;
   size_t mm_scratch_zeroed = 0;
 };
 
@@ -41,62 +41,122 @@ int find_thresholds(CalibCtx* c, int tensors, const int32_t* const* hist_dev, co
                     const float* widths, long long dst_bins, float* thresholds_host, float* kl_host, cudaStream_t s) {
   if (tensors == 0) return B200Q_OK;
   if (dst_bins != 128 && dst_bins != 8) return set_error(B200Q_ERR_INVALID, "find_threshold: dst_bins must be 128 or 8 (asserted by the reference)");
-  std::vector<long long> offs((size_t)tensors + 1, 0);
-  std::vector<float> wfinal((size_t)tensors);
+  // A histogram short enough is searched where it lies (its zero padding is implied by its length); longer ones are
+  // folded into `work` first.
+  std::vector<KldTensor> tab((size_t)tensors);
   std::vector<int> folds((size_t)tensors);
-  long long max_len = 0, max_tmp = 0;
+  std::vector<long long> offs((size_t)tensors);
+  long long max_len = 0, max_tmp = 0, folded = 0;
   for (int t = 0; t < tensors; ++t) {
     if (n_bins[t] < 1 || !hist_dev[t]) return set_error(B200Q_ERR_INVALID, "find_threshold: empty histogram %d", t);
     long long L;
-    fold_plan(n_bins[t], widths[t], dst_bins, &L, &wfinal[(size_t)t], &folds[(size_t)t]);
-    offs[(size_t)t + 1] = offs[(size_t)t] + L;
+    KldTensor& k = tab[(size_t)t];
+    fold_plan(n_bins[t], widths[t], dst_bins, &L, &k.width, &folds[(size_t)t]);
+    k.hist = hist_dev[t];
+    k.n_in = (int)(folds[(size_t)t] ? L : n_bins[t]);
+    k.len = (int)L;
     if (L > max_len) max_len = L;
+    if (folds[(size_t)t]) {
+      offs[(size_t)t] = folded;
+      folded += L;
+    }
     if (folds[(size_t)t] > 1) {
       const long long tmp = pad_to(pad_to(n_bins[t], dst_bins) / 2, dst_bins);
       if (tmp > max_tmp) max_tmp = tmp;
     }
   }
-  B200Q_TRY(c->work.ensure((size_t)offs[(size_t)tensors] * 4));
+  if (folded) B200Q_TRY(c->work.ensure((size_t)folded * 4));
   if (max_tmp) {
     B200Q_TRY(c->work2.ensure((size_t)max_tmp * 4));
     B200Q_TRY(c->stage.ensure((size_t)max_tmp * 4));
   }
-  int* work = c->work.as<int>();
   for (int t = 0; t < tensors; ++t) {
-    int* dst = work + offs[(size_t)t];
-    const long long L = offs[(size_t)t + 1] - offs[(size_t)t];
-    if (folds[(size_t)t] == 0) {
-      CUDA_TRY(cudaMemcpyAsync(dst, hist_dev[t], (size_t)n_bins[t] * 4, cudaMemcpyDeviceToDevice, s));
-      if (L > n_bins[t]) CUDA_TRY(cudaMemsetAsync(dst + n_bins[t], 0, (size_t)(L - n_bins[t]) * 4, s));
-    } else {
-      // fold chain; intermediate results ping-pong between two scratch buffers, the last step lands in `dst`
-      const int* src = hist_dev[t];
-      long long n_in = n_bins[t], cur = pad_to(n_bins[t], dst_bins);
-      int* bufs[2] = {c->work2.as<int>(), c->stage.as<int>()};
-      for (int f = 0; f < folds[(size_t)t]; ++f) {
-        const long long n_out = pad_to(cur / 2, dst_bins);
-        int* out = (f == folds[(size_t)t] - 1) ? dst : bufs[f & 1];
-        B200Q_TRY(fold_launch(src, n_in, out, n_out, s));
-        src = out;
-        n_in = n_out;
-        cur = n_out;
-      }
+    if (folds[(size_t)t] == 0) continue;
+    // fold chain; intermediate results ping-pong between two scratch buffers, the last step lands in `dst`
+    int* dst = c->work.as<int>() + offs[(size_t)t];
+    const int* src = hist_dev[t];
+    long long n_in = n_bins[t], cur = pad_to(n_bins[t], dst_bins);
+    int* bufs[2] = {c->work2.as<int>(), c->stage.as<int>()};
+    for (int f = 0; f < folds[(size_t)t]; ++f) {
+      const long long n_out = pad_to(cur / 2, dst_bins);
+      int* out = (f == folds[(size_t)t] - 1) ? dst : bufs[f & 1];
+      B200Q_TRY(fold_launch(src, n_in, out, n_out, s));
+      src = out;
+      n_in = n_out;
+      cur = n_out;
     }
+    tab[(size_t)t].hist = dst;
   }
-  B200Q_TRY(c->offsets.upload(offs.data(), offs.size() * sizeof(long long), s));
-  B200Q_TRY(c->widths.upload(wfinal.data(), wfinal.size() * sizeof(float), s));
+  B200Q_TRY(c->table.upload(tab.data(), tab.size() * sizeof(KldTensor), s));
   B200Q_TRY(c->thresholds.ensure((size_t)tensors * 4));
-  float* kl_dev = nullptr;
-  if (kl_host) {
-    B200Q_TRY(c->kl.ensure((size_t)tensors * 1024 * 4));
-    kl_dev = c->kl.as<float>();
-  }
-  B200Q_TRY(kld_launch(work, c->offsets.as<long long>(), c->widths.as<float>(), tensors, (int)dst_bins, max_len,
-                       c->thresholds.as<float>(), kl_dev, s));
+  B200Q_TRY(c->kl.ensure((size_t)tensors * 1024 * 4));
+  B200Q_TRY(kld_launch(c->table.as<KldTensor>(), tensors, (int)dst_bins, max_len, c->thresholds.as<float>(), c->kl.as<float>(), s));
   CUDA_TRY(cudaMemcpyAsync(thresholds_host, c->thresholds.p, (size_t)tensors * 4, cudaMemcpyDeviceToHost, s));
   if (kl_host) CUDA_TRY(cudaMemcpyAsync(kl_host, c->kl.p, (size_t)tensors * 1024 * 4, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
   return B200Q_OK;
+}
+
+// Statistics over many tensors: the table (and what follows it) in one upload.
+int upload_table(CalibCtx* c, int tensors, const float* const* x, const int64_t* n_per_sample, int64_t samples, int32_t* const* hist,
+                 const void* tail, size_t tail_bytes, cudaStream_t s, long long* total, long long* chunks) {
+  std::vector<char> packed((size_t)tensors * sizeof(CalibTensor) + tail_bytes);
+  CalibTensor* tab = reinterpret_cast<CalibTensor*>(packed.data());
+  *total = *chunks = 0;
+  for (int t = 0; t < tensors; ++t) {
+    if (!x[t] || n_per_sample[t] < 1) return set_error(B200Q_ERR_INVALID, "calib: tensor %d is empty", t);
+    tab[t].x = x[t];
+    tab[t].hist = hist ? hist[t] : nullptr;
+    tab[t].n = n_per_sample[t];
+    tab[t].first = *total;
+    tab[t].first_chunk = *chunks;
+    *total += n_per_sample[t] * samples;
+    *chunks += minmax_many_chunks(n_per_sample[t], samples);
+  }
+  if (tail_bytes) memcpy(packed.data() + (size_t)tensors * sizeof(CalibTensor), tail, tail_bytes);
+  return c->params.upload(packed.data(), packed.size(), s);
+}
+
+float float_of_ordered(uint32_t u) {
+  const uint32_t b = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
+  float f;
+  memcpy(&f, &b, 4);
+  return f;
+}
+
+// numpy's floor_divide of two positive finite float32 values (the reference's `//`): the quotient from the exact remainder
+float floor_divide_f32(float a, float b) {
+  const float mod = fmodf(a, b);
+  const float div = (a - mod) / b;
+  if (div == 0.f) return 0.f;
+  float fl = floorf(div);
+  if (div - fl > 0.5f) fl += 1.f;
+  return fl;
+}
+
+int histogram_many(CalibCtx* c, int tensors, const float* const* x, const int64_t* n_per_sample, int64_t samples, const float* th_host,
+                   const int32_t* nbins_host, int32_t* const* hist, const int64_t* hist_len, cudaStream_t s) {
+  const size_t rows = (size_t)tensors * (size_t)samples;
+  int fit = 0, max_bins = 0;
+  for (int t = 0; t < tensors; ++t) {
+    if (!hist[t]) return set_error(B200Q_ERR_INVALID, "calib_histogram: null histogram");
+    for (int64_t i = 0; i < samples; ++i) {
+      const int nb = nbins_host[(size_t)t * samples + i];
+      if (nb < 0 || nb > hist_len[t]) return set_error(B200Q_ERR_INVALID, "calib_histogram: nbins[%lld] = %d exceeds the histogram length %lld", (long long)i, nb, (long long)hist_len[t]);
+      if (nb == 1) return set_error(B200Q_ERR_INVALID, "calib_histogram: a histogram needs at least 2 bins");
+      if (nb > max_bins) max_bins = nb;
+      if (nb > fit && nb <= histogram_max_shared_bins()) fit = nb;
+    }
+  }
+  if (max_bins == 0) return B200Q_OK;
+  std::vector<char> tail(rows * 8);   // th | nbins
+  memcpy(tail.data(), th_host, rows * 4);
+  memcpy(tail.data() + rows * 4, nbins_host, rows * 4);
+  long long total, chunks;
+  B200Q_TRY(upload_table(c, tensors, x, n_per_sample, samples, hist, tail.data(), tail.size(), s, &total, &chunks));
+  const char* dev = c->params.as<char>() + (size_t)tensors * sizeof(CalibTensor);
+  return histogram_launch(c->params.as<CalibTensor>(), tensors, samples, total, reinterpret_cast<const float*>(dev),
+                          reinterpret_cast<const int*>(dev + rows * 4), fit ? fit : max_bins, s);
 }
 
 CalibCtx* global_ctx() {
@@ -154,22 +214,91 @@ int b200q_calib_histogram(void* ctx, const float* x_dev, int64_t n_per_sample, i
                           const int32_t* nbins_host, int32_t* hist_dev, int64_t hist_len, void* stream) {
   if (!ctx || !x_dev || !th_host || !nbins_host || !hist_dev || n_per_sample < 1 || samples < 0)
     return set_error(B200Q_ERR_INVALID, "calib_histogram: bad argument");
+  return histogram_many(static_cast<CalibCtx*>(ctx), 1, &x_dev, &n_per_sample, samples, th_host, nbins_host, &hist_dev, &hist_len,
+                        static_cast<cudaStream_t>(stream));
+}
+
+int b200q_calib_minmax_many(void* ctx, int32_t tensors, const float* const* x_dev, const int64_t* n_per_sample, int64_t samples,
+                            float* minmax_host, void* stream) {
+  if (!ctx || tensors < 1 || !x_dev || !n_per_sample || samples < 1 || samples > 0x7fffffffLL || !minmax_host)
+    return set_error(B200Q_ERR_INVALID, "calib_minmax_many: bad argument");
   CalibCtx* c = static_cast<CalibCtx*>(ctx);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int max_bins = 0;
-  for (int64_t i = 0; i < samples; ++i) {
-    if (nbins_host[i] < 0 || nbins_host[i] > hist_len) return set_error(B200Q_ERR_INVALID, "calib_histogram: nbins[%lld] = %d exceeds the histogram length %lld", (long long)i, nbins_host[i], (long long)hist_len);
-    if (nbins_host[i] == 1) return set_error(B200Q_ERR_INVALID, "calib_histogram: a histogram needs at least 2 bins");
-    if (nbins_host[i] > max_bins) max_bins = nbins_host[i];
+  const size_t rows = (size_t)tensors * (size_t)samples;
+  long long total, chunks;
+  B200Q_TRY(upload_table(c, tensors, x_dev, n_per_sample, samples, nullptr, nullptr, 0, s, &total, &chunks));
+  B200Q_TRY(c->mm_out.ensure(rows * 8));
+  uint32_t* lo = c->mm_out.as<uint32_t>();
+  CUDA_TRY(cudaMemsetAsync(lo, 0xff, rows * 4, s));
+  CUDA_TRY(cudaMemsetAsync(lo + rows, 0, rows * 4, s));
+  B200Q_TRY(minmax_many_launch(c->params.as<CalibTensor>(), tensors, samples, chunks, lo, lo + rows, s));
+  std::vector<uint32_t> raw(rows * 2);
+  CUDA_TRY(cudaMemcpyAsync(raw.data(), lo, rows * 8, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaStreamSynchronize(s));
+  for (size_t i = 0; i < rows; ++i) {
+    minmax_host[2 * i] = float_of_ordered(raw[i]);
+    minmax_host[2 * i + 1] = float_of_ordered(raw[rows + i]);
   }
-  if (max_bins == 0) return B200Q_OK;
-  // th | nbins packed in one upload
-  std::vector<char> packed((size_t)samples * 8);
-  memcpy(packed.data(), th_host, (size_t)samples * 4);
-  memcpy(packed.data() + (size_t)samples * 4, nbins_host, (size_t)samples * 4);
-  B200Q_TRY(c->params.upload(packed.data(), packed.size(), s));
-  return histogram_launch(x_dev, n_per_sample, samples, c->params.as<float>(),
-                          reinterpret_cast<const int*>(c->params.as<char>() + (size_t)samples * 4), hist_dev, max_bins, s);
+  return B200Q_OK;
+}
+
+int b200q_calib_histogram_many(void* ctx, int32_t tensors, const float* const* x_dev, const int64_t* n_per_sample, int64_t samples,
+                               const float* th_host, const int32_t* nbins_host, int32_t* const* hist_dev, const int64_t* hist_len,
+                               void* stream) {
+  if (!ctx || tensors < 1 || !x_dev || !n_per_sample || samples < 1 || samples > 0x7fffffffLL || !th_host || !nbins_host || !hist_dev || !hist_len)
+    return set_error(B200Q_ERR_INVALID, "calib_histogram_many: bad argument");
+  return histogram_many(static_cast<CalibCtx*>(ctx), tensors, x_dev, n_per_sample, samples, th_host, nbins_host, hist_dev, hist_len,
+                        static_cast<cudaStream_t>(stream));
+}
+
+int b200q_calib_bin_schedule(b200q_bin_state* state, int32_t tensors, int64_t samples, const float* minmax, int64_t first_sample,
+                             int32_t bin_num, int64_t max_bins, float* th, int32_t* nbins) {
+  if (!state || tensors < 0 || samples < 0 || (tensors > 0 && samples > 0 && (!minmax || !th || !nbins)) || bin_num < 2)
+    return set_error(B200Q_ERR_INVALID, "calib_bin_schedule: bad argument");
+  for (int32_t t = 0; t < tensors; ++t) {
+    b200q_bin_state& st = state[t];
+    for (int64_t i = 0; i < samples; ++i) {
+      const float lo = minmax[((size_t)t * samples + i) * 2], hi = minmax[((size_t)t * samples + i) * 2 + 1];
+      if (lo < st.min) st.min = lo;
+      if (hi > st.max) st.max = hi;
+      const float abs_value = fmaxf(fabsf(st.min), fabsf(st.max));
+      float* const th_i = th + (size_t)t * samples + i;
+      int32_t* const nb_i = nbins + (size_t)t * samples + i;
+      if (fmaxf(fabsf(lo), fabsf(hi)) < 1e-8f) {   // an all-zero activation contributes nothing
+        *th_i = 0.f;
+        *nb_i = 0;
+        continue;
+      }
+      bool moved = false;
+      if (!st.started) {
+        st.th = abs_value;
+        st.bins = bin_num;
+        st.started = 1;
+        moved = true;
+      } else if (abs_value > st.th) {
+        const float old_step = st.th / (float)st.bins;
+        const float grown = floor_divide_f32(abs_value - st.th, old_step) + 1.f;
+        const int64_t inc = grown >= 0.f && grown < 9e18f ? (int64_t)grown : (grown >= 9e18f && grown <= 3.402823e38f ? max_bins + 1 : 0);
+        if (inc + st.bins > max_bins) {
+          st.th = abs_value;
+          st.bins = bin_num;
+          st.last_reset = first_sample + i;
+          for (int64_t j = 0; j < i; ++j) {   // (earlier calls' samples: the caller drops what it counted for them)
+            th[(size_t)t * samples + j] = 0.f;
+            nbins[(size_t)t * samples + j] = 0;
+          }
+        } else {
+          st.th = (float)inc * old_step + st.th;
+          st.bins = inc + st.bins;
+        }
+        moved = true;
+      }
+      if (moved) st.width = st.th / (float)(st.bins - 1);
+      *th_i = st.th;
+      *nb_i = (int32_t)st.bins;
+    }
+  }
+  return B200Q_OK;
 }
 
 void b200q_calib_set_histogram_layout(int32_t mode) { histogram_set_mode(mode); }
@@ -199,14 +328,10 @@ float kl_diversity_hist(int* data, float width, long long num_bins, long long ds
     set_error(B200Q_ERR_UNSUPPORTED, "kl_diversity_hist: more than 1024 candidates");
     return NAN;
   }
-  const long long offs[2] = {0, num_bins};
   float th = NAN;
-  if (c->offsets.upload(offs, sizeof(offs), s) != B200Q_OK || c->widths.upload(&width, 4, s) != B200Q_OK ||
-      c->thresholds.ensure(4) != B200Q_OK)
-    return NAN;
-  if (kld_launch(c->stage.as<int>(), c->offsets.as<long long>(), c->widths.as<float>(), 1, (int)dst_bins, num_bins,
-                 c->thresholds.as<float>(), nullptr, s) != B200Q_OK)
-    return NAN;
+  const KldTensor k{c->stage.as<int>(), (int)num_bins, (int)num_bins, width};
+  if (c->table.upload(&k, sizeof(k), s) != B200Q_OK || c->thresholds.ensure(4) != B200Q_OK || c->kl.ensure(1024 * 4) != B200Q_OK) return NAN;
+  if (kld_launch(c->table.as<KldTensor>(), 1, (int)dst_bins, num_bins, c->thresholds.as<float>(), c->kl.as<float>(), s) != B200Q_OK) return NAN;
   if (cudaMemcpyAsync(&th, c->thresholds.p, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
     cuda_error(cudaGetLastError(), "kl_diversity_hist", __FILE__, __LINE__);
     return NAN;
@@ -237,14 +362,10 @@ float kl_diversity(float* data, long long count, long long num_bins) {
   if (c->stage.ensure((size_t)num_bins * 4) != B200Q_OK) return NAN;
   cudaMemsetAsync(c->stage.p, 0, (size_t)num_bins * 4, s);
   if (kl_raw_histogram_launch(c->work2.as<float>(), count, width, (int)num_bins, c->stage.as<int>(), s) != B200Q_OK) return NAN;
-  const long long offs[2] = {0, num_bins};
   float th = NAN;
-  if (c->offsets.upload(offs, sizeof(offs), s) != B200Q_OK || c->widths.upload(&width, 4, s) != B200Q_OK ||
-      c->thresholds.ensure(4) != B200Q_OK)
-    return NAN;
-  if (kld_launch(c->stage.as<int>(), c->offsets.as<long long>(), c->widths.as<float>(), 1, (int)BINS, num_bins,
-                 c->thresholds.as<float>(), nullptr, s) != B200Q_OK)
-    return NAN;
+  const KldTensor k{c->stage.as<int>(), (int)num_bins, (int)num_bins, width};
+  if (c->table.upload(&k, sizeof(k), s) != B200Q_OK || c->thresholds.ensure(4) != B200Q_OK || c->kl.ensure(1024 * 4) != B200Q_OK) return NAN;
+  if (kld_launch(c->table.as<KldTensor>(), 1, (int)BINS, num_bins, c->thresholds.as<float>(), c->kl.as<float>(), s) != B200Q_OK) return NAN;
   if (cudaMemcpyAsync(&th, c->thresholds.p, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return NAN;
   return th;
 }
