@@ -3,6 +3,7 @@
 // the convolution takes HOST float buffers like top::ConvOp::inference (lib/Dialect/Top/Interfaces/Conv.cpp:222-231).
 #include <string.h>
 
+#include <mutex>
 #include <new>
 
 #include "../../include/b200q.h"
@@ -14,9 +15,62 @@ using namespace b200q;
 
 namespace {
 
+// Scratch of the tensor-core convolutions: stream-ordered allocations from one memory pool per device.  A call's scratch is
+// dead when its kernels are, so the layers of a network use the same few megabytes one after the other (which then stay in
+// the L2), and calls on different streams or threads get different ones.  The pool keeps at most POOL_KEEP bytes between
+// calls and gives everything back with the last handle of its device.
+constexpr uint64_t POOL_KEEP = 256ull << 20;
+constexpr int POOL_DEVICES = 64;
+struct ScratchPools {
+  std::mutex m;
+  cudaMemPool_t pool[POOL_DEVICES] = {};
+  int refs[POOL_DEVICES] = {};
+};
+ScratchPools& scratch_pools() {
+  static ScratchPools* p = new ScratchPools;   // never destroyed: handles may outlive static destruction
+  return *p;
+}
+cudaMemPool_t pool_acquire(int dev) {
+  if (dev < 0 || dev >= POOL_DEVICES) return nullptr;
+  ScratchPools& sp = scratch_pools();
+  std::lock_guard<std::mutex> lock(sp.m);
+  if (!sp.pool[dev]) {   // (the empty pool itself stays: destroying it while frees are still on their way is not worth the care)
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    if (cudaMemPoolCreate(&sp.pool[dev], &props) != cudaSuccess) {
+      cudaGetLastError();
+      sp.pool[dev] = nullptr;
+      return nullptr;
+    }
+    uint64_t keep = POOL_KEEP;
+    cudaMemPoolSetAttribute(sp.pool[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  ++sp.refs[dev];
+  return sp.pool[dev];
+}
+// One handle's share in its device's pool.  Declared before the handle's buffers, so it goes after them: cudaFree has then
+// waited for the handle's kernels, and the scratch they used is free.
+struct PoolRef {
+  cudaMemPool_t pool = nullptr;   // null: no scratch, the tensor-core form is not used
+  int dev = -1;
+  PoolRef() = default;
+  PoolRef(const PoolRef&) = delete;
+  PoolRef& operator=(const PoolRef&) = delete;
+  ~PoolRef() {
+    if (!pool) return;
+    ScratchPools& sp = scratch_pools();
+    std::lock_guard<std::mutex> lock(sp.m);
+    if (--sp.refs[dev] == 0) cudaMemPoolTrimTo(pool, 0);
+  }
+};
+
 struct TopConvHandle {
   TopConvPlan plan{};
+  PoolRef scratch;
   DevBuf wt, ktab, bias, w_stage, x, y, ws;
+  DevBuf planes;                   // the weight as three bf16 planes, where the tensor-core form applies
   bool with_bias = false;
   const float* d_bias = nullptr;   // device face: the caller's
 };
@@ -62,6 +116,11 @@ int b200q_top_conv2d_dev_create(const b200q_top_conv_desc* desc, const float* fi
   int rc = h->wt.ensure((size_t)p.oc * p.K * 4);
   if (rc == B200Q_OK) rc = h->ktab.ensure((size_t)p.K * sizeof(int2));
   if (rc == B200Q_OK) rc = top_conv_prepare(p, filter_oihw, h->wt.as<float>(), h->ktab.as<int2>(), 0);
+  if (rc == B200Q_OK && top_conv_umma_takes(p) && cudaGetDevice(&h->scratch.dev) == cudaSuccess) {
+    if (h->planes.ensure(top_conv_umma_weight_bytes(p)) == B200Q_OK) h->scratch.pool = pool_acquire(h->scratch.dev);
+    else cudaGetLastError();       // no room for the planes: the CUDA-core kernel serves this layer
+    if (h->scratch.pool) rc = top_conv_umma_prepare(p, filter_oihw, h->planes.p, 0);
+  }
   if (rc == B200Q_OK && cudaStreamSynchronize(0) != cudaSuccess) rc = cuda_error(cudaGetLastError(), "sync", __FILE__, __LINE__);
   if (rc != B200Q_OK) {
     delete h;
@@ -79,6 +138,17 @@ int b200q_top_conv2d_dev_run(void* handle, const float* x, float* y, int64_t bat
   int dev = 0, sms = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (h->scratch.pool && p.n > 0 && dev == h->scratch.dev && !(reinterpret_cast<uintptr_t>(x) & 3) && !(reinterpret_cast<uintptr_t>(y) & 15)) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    void* scratch = nullptr;
+    if (cudaMallocFromPoolAsync(&scratch, top_conv_umma_scratch(p, sms), h->scratch.pool, s) == cudaSuccess) {
+      const int rc = top_conv_umma_launch(p, x, h->wt.as<float>(), h->planes.p, h->d_bias, y, scratch, sms, s);
+      const cudaError_t e = cudaFreeAsync(scratch, s);
+      if (rc == B200Q_OK && e != cudaSuccess) return cuda_error(e, "cudaFreeAsync", __FILE__, __LINE__);
+      return rc;
+    }
+    cudaGetLastError();   // no scratch to be had: the CUDA-core kernel needs none
+  }
   p.splits = top_conv_splits(p, sms);
   if (p.splits > 1) B200Q_TRY(h->ws.ensure((size_t)p.splits * p.n * p.oc * p.oh * p.ow * 4));   // grows on the first call of a batch size
   return top_conv_launch(p, x, h->wt.as<float>(), h->ktab.as<int2>(), h->d_bias, y, h->ws.as<float>(), static_cast<cudaStream_t>(stream));
