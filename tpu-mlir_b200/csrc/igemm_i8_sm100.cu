@@ -990,7 +990,14 @@ int igemm_i8_tcgen05_supported(const IGemmProblem& p, const char** why) {
 int igemm_i8_tcgen05_launch(const IGemmProblem& p, const Epilogue& epi, int* status, cudaStream_t stream) {
   const char* why = nullptr;
   if (!igemm_i8_tcgen05_supported(p, &why)) return set_error(B200Q_ERR_UNSUPPORTED, "tcgen05 igemm: %s", why);
-  const int block_n = p.n > 128 ? 256 : (p.n > 64 ? 128 : 64);
+  int dev = 0, sms = 0;
+  CUDA_TRY(cudaGetDevice(&dev));
+  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // Tiles as wide as the product, until they leave more than half of the SMs idle: a CTA's time is what its operand rows
+  // (128 of A and block_n of B per k block) take to come in, so half the width on twice the CTAs is shorter.  (Per-row
+  // parameters are built for the 256-column tile.)
+  int block_n = p.n > 128 ? 256 : (p.n > 64 ? 128 : 64);
+  while (block_n > 64 && !p.per_row_params && 2ll * ((p.rows + BLOCK_M - 1) / BLOCK_M) * ((p.n + block_n - 1) / block_n) <= sms) block_n /= 2;
   const int kb_per_tap = (p.k_per_tap + BLOCK_K - 1) / BLOCK_K;
 
   IGemmArgs a{};
@@ -1064,9 +1071,6 @@ int igemm_i8_tcgen05_launch(const IGemmProblem& p, const Epilogue& epi, int* sta
     a.out_small = out_elems < (1ll << 31);
   }
   // CTA pairs (256-row tiles, cta_group::2) once there is more than one wave of 128-row tiles to share out
-  int dev = 0, sms = 0;
-  CUDA_TRY(cudaGetDevice(&dev));
-  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const long long tiles128 = (long long)((p.rows + BLOCK_M - 1) / BLOCK_M) * ((p.n + block_n - 1) / block_n);
   const bool pair = block_n == 256 && pair_mode_allowed() && tiles128 >= 2ll * sms && p.rows > BLOCK_M;
   // three taps per filter row, one pixel apart, no ragged K block: the taps of a row share one activation block
