@@ -202,12 +202,10 @@ int b200q_top_matmul_f32_dev(const float* x, const float* w_kn, const float* bia
                              int32_t do_relu, float relu_limit, void* stream) {
   if (!x || !w_kn || !y) return set_error(B200Q_ERR_INVALID, "top_matmul_f32_dev: null argument");
   if (M < 0 || K < 1 || N < 1 || M > 0x7fffffffLL || K > 0x7fffffffLL || N > 0x7fffffffLL) return set_error(B200Q_ERR_INVALID, "top_matmul_f32_dev: bad shape");
-  // x[M][K] * w[K][N]: a 1x1 convolution over M one-pixel images; without a table the gather offset of k is k itself
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  TopConvPlan p{};
-  p.n = (int)M; p.ic = (int)K; p.ih = p.iw = p.oh = p.ow = 1; p.oc = (int)N; p.kh = p.kw = p.sh = p.sw = p.dh = p.dw = 1;
-  p.groups = 1; p.icg = (int)K; p.ocg = (int)N; p.K = (int)K; p.do_relu = do_relu ? 1 : 0; p.relu_limit = relu_limit;
-  return top_conv_launch(p, x, w_kn, nullptr, bias, y, nullptr, s);
+  int dev = 0, sms = 0;
+  CUDA_TRY(cudaGetDevice(&dev));
+  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  return top_matmul_launch(x, w_kn, bias, y, (int)M, (int)K, (int)N, do_relu ? 1 : 0, relu_limit, sms, static_cast<cudaStream_t>(stream));
 }
 
 int b200q_top_pool2d_f32_dev(const float* x, float* y, int64_t nc, int32_t ih, int32_t iw, int32_t kh, int32_t kw, int32_t sh,

@@ -13,6 +13,7 @@
 // with a per-k table (offset of (c, kh, kw) inside an image and the two shifts for the border test), the pixel's own
 // decomposition (image, row, column) is computed once per thread.  In NCHW consecutive pixels are consecutive
 // addresses for a fixed k, so both the gather and the store run along the fast axis.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -242,6 +243,73 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, const float* 
     const float bv = bias ? __ldg(bias + (int)(((i4 + e) / ohow) % oc)) : 0.f;
     y[i4 + e] = relu_f(with_bias(a, bv), do_relu, relu_limit);
   }
+}
+
+// y[M][N] = relu(x[M][K] * w[K][N] + bias) where the 128 x 128 tiles of the convolution kernel would leave most SMs idle (a
+// classifier: 32 x 2048 x 1000 has eight of them, each walking all of K: 261 us).  32 x 64 tiles, K shared out over the CTAs
+// of a cluster, which add their partial sums up through distributed shared memory in rank order.  What is left is the
+// latency of one CTA's share of K and reading w once: 261 -> 9 us.
+constexpr int MM_M = 32, MM_N = 64, MM_K = 64, MM_THREADS = 256, MM_CLUSTER = 8;
+__global__ void __launch_bounds__(MM_THREADS) matmul_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                                                                const float* __restrict__ bias, float* __restrict__ y, int M, int K,
+                                                                int N, int do_relu, float relu_limit) {
+  __shared__ __align__(16) float xs[MM_K][MM_M + 2];
+  __shared__ __align__(16) float ws[MM_K][MM_N];
+  __shared__ __align__(16) float part[MM_M][MM_N];
+  const unsigned ranks = gridDim.z, rank = blockIdx.z;   // the cluster spans the grid's z axis
+  const int m0 = blockIdx.y * MM_M, n0 = blockIdx.x * MM_N;
+  const int share = ((K + (int)ranks - 1) / (int)ranks + MM_K - 1) / MM_K * MM_K;
+  const int k_begin = min((long long)K, (long long)rank * share), k_end = min((long long)K, (long long)k_begin + share);
+  const int tid = threadIdx.x, lo = tid & 63, hi = tid >> 6;
+  const int tx = (tid & 15) * 4, ty = (tid >> 4) * 2;
+  float acc[2][4] = {};
+  float rx[8], rw[16];   // the next slice, on its way while this one is multiplied
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int m = m0 + hi + 4 * i, k = k0 + lo;
+      rx[i] = (m < M && k < k_end) ? __ldg(x + (long long)m * K + k) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int k = k0 + hi + 4 * i, n = n0 + lo;
+      rw[i] = (n < N && k < k_end) ? __ldg(w + (long long)k * N + n) : 0.f;
+    }
+  };
+  if (k_begin < k_end) fetch(k_begin);
+  for (int k0 = k_begin; k0 < k_end; k0 += MM_K) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) xs[lo][hi + 4 * i] = rx[i];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) ws[hi + 4 * i][lo] = rw[i];
+    __syncthreads();
+    if (k0 + MM_K < k_end) fetch(k0 + MM_K);
+#pragma unroll 16
+    for (int k = 0; k < MM_K; ++k) {
+      const float2 a = *reinterpret_cast<const float2*>(&xs[k][ty]);
+      const float4 b = *reinterpret_cast<const float4*>(&ws[k][tx]);
+      const float av[2] = {a.x, a.y}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(&part[ty + i][tx]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  // this CTA finishes its share of the tile's elements
+  const int per = MM_M * MM_N / (int)ranks;
+  for (int e = (int)rank * per + tid; e < ((int)rank + 1) * per; e += MM_THREADS) {
+    const int m = m0 + e / MM_N, n = n0 + e % MM_N;
+    if (m >= M || n >= N) continue;
+    float v = 0.f;
+    for (unsigned r = 0; r < ranks; ++r) v += cluster.map_shared_rank(&part[0][0], r)[e];
+    y[(long long)m * N + n] = relu_f(v + (bias ? __ldg(bias + n) : 0.f), do_relu, relu_limit);
+  }
+  cluster.sync();   // nobody leaves while its sums are being read
 }
 
 // (c, kh, kw) of every k: offset inside an image and the two border shifts
@@ -1025,6 +1093,37 @@ int top_conv_launch(const TopConvPlan& plan, const float* x, const float* wt, co
   }
   CUDA_TRY(cudaGetLastError());
   if (p.splits > 1) return top_conv_reduce_launch(workspace, bias, y, P * p.oc, p.splits, p.oc, p.oh * p.ow, p.do_relu, p.relu_limit, 0.f, s);
+  return B200Q_OK;
+}
+
+// 128 x 128 tiles for at most half of the SMs: the split form.  Above, the convolution kernel's larger tiles, which load less
+// per product, keep enough SMs busy.  (K beyond 2^30: its index arithmetic stays in 32 bits.)
+int top_matmul_launch(const float* x, const float* w_kn, const float* bias, float* y, int M, int K, int N, int do_relu, float relu_limit,
+                      int sms, cudaStream_t s) {
+  const long long tiles = (long long)((M + 127) / 128) * ((N + 127) / 128);
+  if (M == 0 || tiles * 2 > sms || K > (1 << 30)) {
+    // a 1x1 convolution over M one-pixel images; without a table the gather offset of k is k itself
+    TopConvPlan p{};
+    p.n = M; p.ic = K; p.ih = p.iw = p.oh = p.ow = 1; p.oc = N; p.kh = p.kw = p.sh = p.sw = p.dh = p.dw = 1;
+    p.groups = 1; p.icg = K; p.ocg = N; p.K = K; p.do_relu = do_relu; p.relu_limit = relu_limit; p.splits = 1;
+    return top_conv_launch(p, x, w_kn, nullptr, bias, y, nullptr, s);
+  }
+  if ((reinterpret_cast<uintptr_t>(x) & 3) || (reinterpret_cast<uintptr_t>(w_kn) & 15) || (reinterpret_cast<uintptr_t>(y) & 15))
+    return set_error(B200Q_ERR_INVALID, "top matmul: operands must be 16-byte aligned");
+  unsigned ranks = 1;
+  while (ranks < MM_CLUSTER && (long long)ranks * 2 * MM_K <= K) ranks *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((N + MM_N - 1) / MM_N), (unsigned)((M + MM_M - 1) / MM_M), ranks);
+  cfg.blockDim = dim3(MM_THREADS);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = ranks;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, matmul_f32_kernel, x, w_kn, bias, y, M, K, N, do_relu, relu_limit));
   return B200Q_OK;
 }
 

@@ -17,8 +17,7 @@ struct TopConvPlan {
 
 // One-time: OIHW weight -> [groups][K][ocg], and the per-k gather table (K entries).
 int top_conv_prepare(const TopConvPlan& p, const float* w_oihw, float* wt, int2* ktab, cudaStream_t s);
-// y[n][oc][oh][ow] = relu(conv(x[n][ic][ih][iw]) + bias); wt / ktab from top_conv_prepare.  A matrix product
-// y[M][N] = x[M][K] * w[K][N] is the case ih = iw = kh = kw = 1 with wt = w and ktab = null.
+// y[n][oc][oh][ow] = relu(conv(x[n][ic][ih][iw]) + bias); wt / ktab from top_conv_prepare.
 // p.splits > 1: `workspace` holds p.splits x (n * oc * oh * ow) floats; every split writes its partial sums there and a
 // second kernel adds them in split order (deterministic) with the bias and the ReLU.
 int top_conv_launch(const TopConvPlan& p, const float* x, const float* wt, const int2* ktab, const float* bias, float* y,
@@ -36,6 +35,9 @@ int top_conv_umma_prepare(const TopConvPlan& p, const float* w_oihw, void* plane
 size_t top_conv_umma_scratch(const TopConvPlan& p, int sms);
 int top_conv_umma_launch(const TopConvPlan& p, const float* x, const float* wt, const void* w_planes, const float* bias, float* y,
                          void* scratch, int sms, cudaStream_t s);
+// y[M][N] = relu(x[M][K] * w[K][N] + bias)
+int top_matmul_launch(const float* x, const float* w_kn, const float* bias, float* y, int M, int K, int N, int do_relu, float relu_limit,
+                      int sms, cudaStream_t s);
 int top_pool2d_launch(const float* x, float* y, long long nc, int ih, int iw, int oh, int ow, int kh, int kw, int sh, int sw,
                       int pht, int phb, int pwl, int pwr, bool is_max, bool count_include_pad, bool do_relu, float relu_limit,
                       cudaStream_t s);
