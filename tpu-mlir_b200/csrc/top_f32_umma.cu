@@ -6,11 +6,11 @@
 // fp32 accumulator whose rounding is coarser than an FMA's, so no accumulator lives longer than 64 products deep: the
 // epilogue warps take it out of tensor memory after every 64 k and add it to their own fp32 sum, rounded to nearest.
 // Against 64-bit sums the result is closer than a serial chain of fp32 FMAs: relative error (2-norm) 4.9e-8 to 1.2e-7 over
-// ResNet-50's layers at batch 32 where the CUDA-core kernel has 1.0e-7 to 3.0e-7, whole network 7.9e-7 against 8.0e-7.
+// ResNet-50's layers at batch 32 where the CUDA-core kernel has 1.0e-7 to 3.0e-7; the whole network's is no larger either.
 //
 // A k chunk of 64 costs 24 MMAs of 128 x BN x 16, a sixth of the bf16 rate: about 260 TFLOP/s of fp32 products where the
 // CUDA cores have 74.  Measured at batch 32: 3x3 128 channels 28x28 210 -> 63 us (117 TFLOP/s), 3x3 256 channels 14x14 198 ->
-// 59 us, 3x3 64 channels 56x56 287 -> 85 us, 1x1 64 to 256 channels 107 -> 69 us.  Two kernels per call:
+// 59 us, 3x3 64 channels 56x56 287 -> 85 us, 1x1 64 to 256 channels 107 -> 54 us.  Two kernels per call:
 //   split_f32_kernel   NCHW fp32 -> three bf16 planes [rows][channels].  Stride 1: rows are the pixels of the padded image,
 //                      and the rows of a filter tap are the same rows shifted (one TMA box per tap, no im2col).  Other
 //                      strides: rows are the output pixels, one channel run per tap.  10 bytes moved per element.
@@ -431,6 +431,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           const float v = s + fmaf(s, gain, __shfl_sync(0xffffffffu, bias[i], j));
           if (valid && i * 32 + j < ncols) *o = relu ? fminf(fmaxf(v, 0.f), ceiling) : v;
           o += ohow;
+          asm volatile("" : "+l"(o));   // one running address: 64 of them kept ahead spilled the sums
         }
       }
       // the rare ones, and everything if a wait ran out (the sums are lost, and say so)
@@ -492,8 +493,10 @@ struct UmmaChoice {
 };
 
 // Tile form and K splits of a launch over `images` images, by a model in nanoseconds.  A chunk costs what its operands cost
-// to bring in (75 bytes per ns and SM, measured) or its 24 MMAs, whichever is more; a round of tiles costs its chunks plus
-// 2 us for the pipeline's start and the stores; partial sums cost a launch and a pass over the output's planes.
+// to bring in (75 bytes per ns and SM, measured) or its 24 MMAs, whichever is more.  These read both operands from shared
+// memory, which sets their pace (128 bytes per clock: 62 clocks measured at 256 x 128 x 16 where the tensor pipe needs 32), so
+// that 256 channels cost little more than 128.  A round of tiles costs its chunks, or its stores, plus 1.5 us for the
+// pipeline's start; partial sums cost a launch and a pass over the output's planes.
 UmmaChoice choose(const TopConvPlan& p, int images, int sms) {
   const bool shifted = shifted_rows(p);
   const long long rows = shifted ? (long long)images * (p.oh + (p.kh - 1) * p.dh) * (p.ow + (p.kw - 1) * p.dw) : (long long)images * p.oh * p.ow;
@@ -509,10 +512,12 @@ UmmaChoice choose(const TopConvPlan& p, int images, int sms) {
     const int tile_m = pair ? 2 * TILE_M : TILE_M;
     const int m_tiles = (int)((rows + tile_m - 1) / tile_m), n_tiles = (p.oc + bn - 1) / bn;
     const double bytes = 3.0 * CHUNK_BYTES * ((double)TILE_M / best.share + (pair ? bn / 2 : bn));
-    const double mma = bn * (pair ? 1.6 : 3.2) * 2, chunk = bytes / 75.0 > mma ? bytes / 75.0 : mma;
+    const double mma = bn == 64 ? 600 : (bn == 128 ? 800 : 1100), chunk = bytes / 75.0 > mma ? bytes / 75.0 : mma;
+    const double store = TILE_M * bn * 4.0 / 20.0;
     for (int sp = 1; sp <= 8 && sp <= best.units; ++sp) {
       const long long tiles = (long long)m_tiles * n_tiles * sp, slots = pair ? sms / 2 : sms;
-      double cost = (double)((tiles + slots - 1) / slots) * ((best.units + sp - 1) / sp * best.share * chunk + 2000.0);
+      const double k_time = (best.units + sp - 1) / sp * best.share * chunk;
+      double cost = (double)((tiles + slots - 1) / slots) * ((k_time > store ? k_time : store) + 1500.0);
       if (sp > 1) cost += 3000.0 + (2.0 * sp + 1) * 4.0 * images * p.oc * p.oh * p.ow / 5000.0;
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
