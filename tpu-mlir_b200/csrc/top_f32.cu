@@ -5,8 +5,9 @@
 // of lib/Support/Dnnl/Pool.cpp: pad value -inf for max, count_include_pad for avg), top::ReluOp (Relu.cpp:17-24 over
 // function_relu, lib/Support/MathUtils.cpp:891-903).  Tensors are NCHW fp32 like the interpreter's buffers.
 //
-// The convolution is an implicit GEMM on the CUDA cores in full fp32 (calibration statistics should not depend on a
-// reduced-precision product): C[co][pixel] = sum_k Wt[k][co] * X[k][pixel], k = (c, kh, kw).  A block computes 128 (or
+// Convolutions with 32 channels or more on both sides and no groups run on the tensor cores (top_f32_umma.cu).  The others
+// are an implicit GEMM on the CUDA cores in full fp32 (calibration statistics should not depend on a reduced-precision
+// product): C[co][pixel] = sum_k Wt[k][co] * X[k][pixel], k = (c, kh, kw).  A block computes 128 (or
 // 64) output channels x 128 pixels, K in slices of 8 through a four-stage ring in shared memory; a thread owns 8 x 8 (4 x 8)
 // results; the tiles travel by cp.async, three slices ahead.  The weight is kept transposed [K][oc] so its tile loads
 // are contiguous; the activation tile is gathered
@@ -248,7 +249,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, const float* 
 // y[M][N] = relu(x[M][K] * w[K][N] + bias) where the 128 x 128 tiles of the convolution kernel would leave most SMs idle (a
 // classifier: 32 x 2048 x 1000 has eight of them, each walking all of K: 261 us).  32 x 64 tiles, K shared out over the CTAs
 // of a cluster, which add their partial sums up through distributed shared memory in rank order.  What is left is the
-// latency of one CTA's share of K and reading w once: 261 -> 9 us.
+// latency of one CTA's share of K and reading w once: 261 -> 18 us.
 constexpr int MM_M = 32, MM_N = 64, MM_K = 64, MM_THREADS = 256, MM_CLUSTER = 8;
 __global__ void __launch_bounds__(MM_THREADS) matmul_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                 const float* __restrict__ bias, float* __restrict__ y, int M, int K,
@@ -331,19 +332,35 @@ __global__ void conv_wt_kernel(const float* __restrict__ w, float* __restrict__ 
   wt[i] = w[((size_t)g * ocg + co) * K + k];
 }
 
-__global__ void pool2d_f32_kernel(const float* __restrict__ x, float* __restrict__ y, long long total, int ih, int iw, int oh,
+// One thread per output.  I: the outputs' index type (32 bits where they fit: the three divisions that take an index apart
+// were most of the instructions).  K3: a 3 x 3 window, whose nine loads are all on their way before the first is used.
+// 32 x 64 x 112 x 112 to 56 x 56: 67 -> 38 us; the 128 MB that it moves would take 20.
+template <typename I, bool K3>
+__global__ void pool2d_f32_kernel(const float* __restrict__ x, float* __restrict__ y, I total, int ih, int iw, int oh,
                                   int ow, int kh, int kw, int sh, int sw, int pht, int pwl, int is_max,
                                   int count_include_pad, int phb, int pwr, int do_relu, float relu_limit) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
-  const int wo = (int)(i % ow);
-  const long long r = i / ow;
-  const int ho = (int)(r % oh);
-  const long long nc = r / oh;
-  const float* src = x + nc * ih * iw;
+  const I r = i / (I)ow;
+  const int wo = (int)(i - r * (I)ow);
+  const I nc = r / (I)oh;
+  const int ho = (int)(r - nc * (I)oh);
+  const float* src = x + (long long)nc * ih * iw;
   const int h0 = ho * sh - pht, w0 = wo * sw - pwl;
   float acc = is_max ? -INFINITY : 0.f;
   int inside = 0;
+  if (K3) {
+    float v[9];
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      const int h = h0 + t / 3, w = w0 + t % 3;
+      v[t] = ((unsigned)h < (unsigned)ih && (unsigned)w < (unsigned)iw) ? __ldg(src + (size_t)h * iw + w) : acc;   // (x + 0, max(x, -inf): no change)
+    }
+#pragma unroll
+    for (int t = 0; t < 9; ++t) acc = is_max ? fmaxf(acc, v[t]) : acc + v[t];
+    inside = (min(h0 + 3, ih) - max(h0, 0)) * (min(w0 + 3, iw) - max(w0, 0));
+    if (h0 >= ih || w0 >= iw || h0 <= -3 || w0 <= -3) inside = 0;
+  } else
   for (int a = 0; a < kh; ++a) {
     const int h = h0 + a;
     if ((unsigned)h >= (unsigned)ih) continue;
@@ -1140,9 +1157,18 @@ int top_pool2d_launch(const float* x, float* y, long long nc, int ih, int iw, in
                       cudaStream_t s) {
   const long long total = nc * oh * ow;
   if (total == 0) return B200Q_OK;
-  pool2d_f32_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(x, y, total, ih, iw, oh, ow, kh, kw, sh, sw, pht, pwl,
-                                                                    is_max ? 1 : 0, count_include_pad ? 1 : 0, phb, pwr,
-                                                                    do_relu ? 1 : 0, relu_limit);
+  const unsigned blocks = (unsigned)((total + 255) / 256);
+  const bool k3 = kh == 3 && kw == 3;
+  auto launch = [&](auto kernel, auto count) {
+    kernel<<<blocks, 256, 0, s>>>(x, y, count, ih, iw, oh, ow, kh, kw, sh, sw, pht, pwl, is_max ? 1 : 0, count_include_pad ? 1 : 0, phb, pwr,
+                                  do_relu ? 1 : 0, relu_limit);
+  };
+  if (total < (1ll << 31)) {
+    if (k3) launch(pool2d_f32_kernel<unsigned, true>, (unsigned)total);
+    else launch(pool2d_f32_kernel<unsigned, false>, (unsigned)total);
+  } else {
+    launch(pool2d_f32_kernel<long long, false>, total);
+  }
   CUDA_TRY(cudaGetLastError());
   return B200Q_OK;
 }
