@@ -994,10 +994,10 @@ int igemm_i8_tcgen05_launch(const IGemmProblem& p, const Epilogue& epi, int* sta
   CUDA_TRY(cudaGetDevice(&dev));
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   // Tiles as wide as the product, until they leave more than half of the SMs idle: a CTA's time is what its operand rows
-  // (128 of A and block_n of B per k block) take to come in, so half the width on twice the CTAs is shorter.  (Per-row
-  // parameters are built for the 256-column tile.)
+  // (128 of A and block_n of B per k block) take to come in, so half the width on twice the CTAs is shorter
+  // (512 x 1024 x 1024: 12.3 -> 8.2 us on 64 instead of 16 CTAs).
   int block_n = p.n > 128 ? 256 : (p.n > 64 ? 128 : 64);
-  while (block_n > 64 && !p.per_row_params && 2ll * ((p.rows + BLOCK_M - 1) / BLOCK_M) * ((p.n + block_n - 1) / block_n) <= sms) block_n /= 2;
+  while (block_n > 64 && 2ll * ((p.rows + BLOCK_M - 1) / BLOCK_M) * ((p.n + block_n - 1) / block_n) <= sms) block_n /= 2;
   const int kb_per_tap = (p.k_per_tap + BLOCK_K - 1) / BLOCK_K;
 
   IGemmArgs a{};
@@ -1110,7 +1110,9 @@ int igemm_i8_tcgen05_launch(const IGemmProblem& p, const Epilogue& epi, int* sta
   const int slots = pair ? sms / 2 : sms;
   const int workers = tiles < slots ? tiles : slots;
   if (p.per_row_params) {
-    if (a.bf16 || block_n != 256) return set_error(B200Q_ERR_UNSUPPORTED, "igemm: per-row parameters need the 256-column tile");
+    if (a.bf16 || p.n <= 128) return set_error(B200Q_ERR_UNSUPPORTED, "igemm: per-row parameters need more than 128 columns of 8-bit operands");
+    if (block_n == 128) return launch_per_row<128, 6, false>(ta, tb, a, workers, stream);
+    if (block_n == 64) return launch_per_row<64, 8, false>(ta, tb, a, workers, stream);
     return pair ? launch_per_row<256, 6, true>(ta, tb, a, workers, stream) : launch_per_row<256, 4, false>(ta, tb, a, workers, stream);
   }
   if (tapfuse) return launch_dialect<256, 3, true, 3>(ta, tb, a, workers, stream);
