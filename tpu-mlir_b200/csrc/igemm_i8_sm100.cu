@@ -993,11 +993,12 @@ int igemm_i8_tcgen05_launch(const IGemmProblem& p, const Epilogue& epi, int* sta
   int dev = 0, sms = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // Tiles as wide as the product, until they leave more than half of the SMs idle: a CTA's time is what its operand rows
+  // Tiles as wide as the product, until they leave two thirds of the SMs idle: a CTA's time is what its operand rows
   // (128 of A and block_n of B per k block) take to come in, so half the width on twice the CTAs is shorter
-  // (512 x 1024 x 1024: 12.3 -> 8.2 us on 64 instead of 16 CTAs).
+  // (512 x 1024 x 1024: 12.3 -> 8.2 us on 64 instead of 16 CTAs).  With the line at half of the SMs ResNet-50 lost 0.5 % at
+  // 93 images (the second tile's rows come over the L2 that the kernels around it need too) and won 1.6 % at 23.
   int block_n = p.n > 128 ? 256 : (p.n > 64 ? 128 : 64);
-  while (block_n > 64 && 2ll * ((p.rows + BLOCK_M - 1) / BLOCK_M) * ((p.n + block_n - 1) / block_n) <= sms) block_n /= 2;
+  while (block_n > 64 && 3ll * ((p.rows + BLOCK_M - 1) / BLOCK_M) * ((p.n + block_n - 1) / block_n) <= sms) block_n /= 2;
   const int kb_per_tap = (p.k_per_tap + BLOCK_K - 1) / BLOCK_K;
 
   IGemmArgs a{};
