@@ -14,7 +14,7 @@ from tpu_mlir_b200.ops import Conv2DOp  # noqa: E402
 ptr = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
 
 
-@pytest.mark.parametrize("M,N", [(1, 65), (128, 129), (130, 257), (513, 1000), (4736, 512), (4737, 512), (2368, 1024), (2369, 1025)])
+@pytest.mark.parametrize("M,N", [(1, 65), (128, 129), (130, 257), (513, 1000), (3072, 512), (3073, 512), (4736, 512), (4737, 512), (2368, 1024), (2369, 1025)])
 @pytest.mark.parametrize("qdm", [False, True])
 def test_matmul(M, N, qdm):
     K = 144
