@@ -219,11 +219,10 @@ __global__ void __launch_bounds__(CONV_THREADS) conv2d_f32_kernel(const float* _
   }
 }
 
-// y = relu(t + t * gain + bias), t the sum over the splits' planes in plane order: 4 outputs per thread (count is a multiple of 4 or the
+// y = relu(sum over the splits' planes, in plane order, + bias): 4 outputs per thread (count is a multiple of 4 or the
 // tail runs element by element)
 __global__ void splitk_reduce_kernel(const float* __restrict__ ws, const float* __restrict__ bias, float* __restrict__ y,
-                                     long long count, int splits, int oc, int ohow, int do_relu, float relu_limit, float gain) {
-  auto with_bias = [&](float t, float b) { return t + (gain != 0.f ? fmaf(t, gain, b) : b); };
+                                     long long count, int splits, int oc, int ohow, int do_relu, float relu_limit) {
   const long long i4 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= count) return;
   const int n = (int)min((long long)4, count - i4);
@@ -234,15 +233,15 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, const float* 
       v[0] += u.x; v[1] += u.y; v[2] += u.z; v[3] += u.w;
     }
     const float bv = bias ? __ldg(bias + (int)((i4 / ohow) % oc)) : 0.f;   // the four share a channel: ohow % 4 == 0
-    *reinterpret_cast<float4*>(y + i4) = make_float4(relu_f(with_bias(v[0], bv), do_relu, relu_limit), relu_f(with_bias(v[1], bv), do_relu, relu_limit),
-                                                     relu_f(with_bias(v[2], bv), do_relu, relu_limit), relu_f(with_bias(v[3], bv), do_relu, relu_limit));
+    *reinterpret_cast<float4*>(y + i4) = make_float4(relu_f(v[0] + bv, do_relu, relu_limit), relu_f(v[1] + bv, do_relu, relu_limit),
+                                                     relu_f(v[2] + bv, do_relu, relu_limit), relu_f(v[3] + bv, do_relu, relu_limit));
     return;
   }
   for (int e = 0; e < n; ++e) {
     float a = 0.f;
     for (int s = 0; s < splits; ++s) a += __ldg(ws + (size_t)s * count + i4 + e);
     const float bv = bias ? __ldg(bias + (int)(((i4 + e) / ohow) % oc)) : 0.f;
-    y[i4 + e] = relu_f(with_bias(a, bv), do_relu, relu_limit);
+    y[i4 + e] = relu_f(a + bv, do_relu, relu_limit);
   }
 }
 
@@ -1109,7 +1108,7 @@ int top_conv_launch(const TopConvPlan& plan, const float* x, const float* wt, co
     else conv2d_f32_kernel<64, 0><<<grid, CONV_THREADS, 0, s>>>(x, wt, ktab, bias, out, p);
   }
   CUDA_TRY(cudaGetLastError());
-  if (p.splits > 1) return top_conv_reduce_launch(workspace, bias, y, P * p.oc, p.splits, p.oc, p.oh * p.ow, p.do_relu, p.relu_limit, 0.f, s);
+  if (p.splits > 1) return top_conv_reduce_launch(workspace, bias, y, P * p.oc, p.splits, p.oc, p.oh * p.ow, p.do_relu, p.relu_limit, s);
   return B200Q_OK;
 }
 
@@ -1145,9 +1144,9 @@ int top_matmul_launch(const float* x, const float* w_kn, const float* bias, floa
 }
 
 int top_conv_reduce_launch(const float* planes, const float* bias, float* y, long long count, int splits, int oc, int ohow, int do_relu,
-                           float relu_limit, float gain, cudaStream_t s) {
+                           float relu_limit, cudaStream_t s) {
   const long long vecs = (count + 3) / 4;
-  splitk_reduce_kernel<<<(unsigned)((vecs + 255) / 256), 256, 0, s>>>(planes, bias, y, count, splits, oc, ohow, do_relu, relu_limit, gain);
+  splitk_reduce_kernel<<<(unsigned)((vecs + 255) / 256), 256, 0, s>>>(planes, bias, y, count, splits, oc, ohow, do_relu, relu_limit);
   CUDA_TRY(cudaGetLastError());
   return B200Q_OK;
 }

@@ -23,9 +23,9 @@ int top_conv_prepare(const TopConvPlan& p, const float* w_oihw, float* wt, int2*
 int top_conv_launch(const TopConvPlan& p, const float* x, const float* wt, const int2* ktab, const float* bias, float* y,
                     float* workspace, cudaStream_t s);
 int top_conv_splits(const TopConvPlan& p, int sms);
-// y = relu(t + t * gain + bias), t the sum of the `splits` planes of `count` floats, in order
+// y = relu(t + bias), t the sum of the `splits` planes of `count` floats, in order
 int top_conv_reduce_launch(const float* planes, const float* bias, float* y, long long count, int splits, int oc, int ohow, int do_relu,
-                           float relu_limit, float gain, cudaStream_t s);
+                           float relu_limit, cudaStream_t s);
 // The same convolution on the tensor cores (top_f32_umma.cu).  takes: whether a plan of one image or more qualifies; prepare:
 // once per handle, the weight's bf16 planes (weight_bytes of them); launch: `scratch` holds top_conv_umma_scratch bytes and is
 // free again when the stream has passed the call.

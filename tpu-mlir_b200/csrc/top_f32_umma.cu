@@ -1,16 +1,21 @@
 // fp32 convolution of the Top dialect on the tensor cores: every fp32 operand as the sum of three bf16 numbers.
 //
-// A float splits exactly into hi + mid + lo (8 significant bits each, round to nearest), a product of two such sums into
-// nine bf16 products that are exact in fp32.  Six of them are multiplied (hi*lo, lo*hi, mid*mid, hi*mid, mid*hi, hi*hi, the
-// smallest first); the three left out are below 2^-25 of the product, half an fp32 rounding.  The tensor core adds into an
-// fp32 accumulator whose rounding is coarser than an FMA's, so no accumulator lives longer than 64 products deep: the
-// epilogue warps take it out of tensor memory after every 64 k and add it to their own fp32 sum, rounded to nearest.
-// Against 64-bit sums the result is closer than a serial chain of fp32 FMAs: relative error (2-norm) 4.9e-8 to 1.2e-7 over
-// ResNet-50's layers at batch 32 where the CUDA-core kernel has 1.0e-7 to 3.0e-7; the whole network's is no larger either.
+// A float splits exactly into hi + mid + lo (6, 8 and 8 significant bits, round to nearest), a product of two such sums into
+// nine bf16 products that are exact in fp32.  Eight of them are multiplied; the ninth, lo*lo, is below 2^-30 of the product.
+// The tensor core adds 16 products and its fp32 accumulator exactly and then cuts the sum off at 24 bits.  What that loses has
+// the sign of the sum, so that it would add up over a network's layers; three things keep it small:
+//   - no accumulator lives longer than 64 products deep: the epilogue warps take it out of tensor memory after every 64 k and
+//     add it to their own fp32 sum, rounded to nearest;
+//   - hi*hi has an accumulator of its own, so that it does not cut off the low bits of the seven smaller products;
+//   - hi has 6 bits instead of the 8 that bf16 holds: a product of 12 bits loses nothing until it is 2^-12 of the sum.
+// Sums that are exact in fp32 stay exact (integers, one-hot filters).  Against 64-bit sums the result is closer than a serial
+// chain of fp32 FMAs: relative error (2-norm) 2.9e-8 to 9.9e-8 over ResNet-50's layers where the CUDA-core kernel has 1.0e-7
+// to 3.1e-7, mean error in the sum's own direction 3e-9 to 4e-9 (4.8e-8 with 8-bit hi parts in one accumulator, 2.7e-8 in two,
+// 5e-9 with an accumulator for every 16 k, which is slower); whole network 3.2e-7 against 8.0e-7.
 //
-// A k chunk of 64 costs 24 MMAs of 128 x BN x 16, a sixth of the bf16 rate: about 260 TFLOP/s of fp32 products where the
-// CUDA cores have 74.  Measured at batch 32: 3x3 128 channels 28x28 210 -> 63 us (117 TFLOP/s), 3x3 256 channels 14x14 198 ->
-// 59 us, 3x3 64 channels 56x56 287 -> 85 us, 1x1 64 to 256 channels 107 -> 54 us.  Two kernels per call:
+// A k chunk of 64 costs 32 MMAs of 128 x BN x 16, an eighth of the bf16 rate: about 200 TFLOP/s of fp32 products where the
+// CUDA cores have 74.  Measured at batch 32: 3x3 128 channels 28x28 203 -> 72 us (102 TFLOP/s), 3x3 256 channels 14x14 196 ->
+// 68 us, 3x3 64 channels 56x56 285 -> 100 us, 1x1 64 to 256 channels 103 -> 52 us.  Two kernels per call:
 //   split_f32_kernel   NCHW fp32 -> three bf16 planes [rows][channels].  Stride 1: rows are the pixels of the padded image,
 //                      and the rows of a filter tap are the same rows shifted (one TMA box per tap, no im2col).  Other
 //                      strides: rows are the output pixels, one channel run per tap.  10 bytes moved per element.
@@ -35,14 +40,11 @@ namespace {
 
 constexpr int TILE_M = 128;                    // rows per CTA
 constexpr int CHUNK = 64;                      // k per accumulator: one 128-byte row of bf16
+constexpr int PARTS = 2;                       // accumulators of a chunk: the seven small products, hi * hi
 constexpr int CHUNK_BYTES = CHUNK * 2;
 constexpr int A_STAGES = 2;
 constexpr int MAX_SHARE = 3;
 constexpr uint64_t WAIT_BUDGET_NS = 2000000000ull;
-// The tensor core's accumulation cuts off instead of rounding: a chunk's sum comes out smaller in magnitude by 4.7e-8 of
-// itself on average (measured against 64-bit sums, K = 64 to 4608; half a unit in the last place).  One layer's share is
-// below its rounding noise, but it has the same sign in every layer; the stored result has it added back.
-constexpr float TRUNCATION = 4.7e-8f;
 
 // BN: channels of a tile.  PAIR: two CTAs of a cluster compute 256 rows x BN channels (tcgen05 cta_group::2); each loads its
 // own 128 rows of A and half of B.
@@ -65,9 +67,12 @@ struct UmmaLayout {
   static constexpr int THREADS = 96 + 32 * EPI_WARPS;
 };
 
-// x = h + m + l, each rounded to bf16 to nearest: exact for every float whose low part is not subnormal
+// x = h + m + l, h rounded to nearest to 6 significant bits, m and l to bf16's 8: 18 bits are left for m, 9 of them and a sign
+// (or 2^8) for l.  Exact for every float whose low part is not subnormal.
 __device__ __forceinline__ void split3(float x, uint16_t& h, uint16_t& m, uint16_t& l) {
-  const __nv_bfloat16 bh = __float2bfloat16_rn(x);
+  const uint32_t u = __float_as_uint(x);
+  const __nv_bfloat16 bh = (u & 0x7f800000u) == 0x7f800000u ? __float2bfloat16_rn(x)
+                                                            : __ushort_as_bfloat16((unsigned short)(((u + 0x20000u) & 0xfffc0000u) >> 16));
   const float r1 = x - __bfloat162float(bh);
   const __nv_bfloat16 bm = __float2bfloat16_rn(r1);
   const float r2 = r1 - __bfloat162float(bm);
@@ -328,30 +333,38 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         for (int u = u0; u < u1 && ok; ++u) {
           ok = ptx::mbar_wait_bounded_fast<20>(full_a(sa), pa, abort_flag, 3, WAIT_BUDGET_NS);
           for (int t = 0; t < share && ok; ++t) {
-            ok = ptx::mbar_wait_bounded_fast<20>(tmem_empty_bar(buf), buf_phase ^ 1u, abort_flag, 4, WAIT_BUDGET_NS) &&
-                 ptx::mbar_wait_bounded_fast<20>(full_b(sb), pb, abort_flag, 5, WAIT_BUDGET_NS);
-            if (!ok) break;
-            ptx::tc_fence_after_sync();
+            ok = ptx::mbar_wait_bounded_fast<20>(full_b(sb), pb, abort_flag, 5, WAIT_BUDGET_NS);
             // tap t reads the block from row t on: the swizzle follows the address bits, only the start moves
             const uint32_t al = a_lo0 + (uint32_t)(sa * (L::A_BYTES >> 4) + t * (CHUNK_BYTES >> 4));
             const uint32_t bl = b_lo0 + (uint32_t)(sb * (L::B_BYTES >> 4));
-            const uint32_t d = tmem_base + (uint32_t)(buf * BN);
-            mma(d, al, bl + 2 * BP, 0u);        // hi * lo
-            mma(d, al + 2 * AP, bl, 1u);        // lo * hi
-            mma(d, al + AP, bl + BP, 1u);       // mid * mid
-            mma(d, al, bl + BP, 1u);            // hi * mid
-            mma(d, al + AP, bl, 1u);            // mid * hi
-            mma(d, al, bl, 1u);                 // hi * hi
-            commit(empty_b(sb));
-            if (t == share - 1) commit(empty_a(sa));
-            commit(tmem_full_bar(buf));
+#pragma unroll
+            for (int part = 0; part < PARTS && ok; ++part) {
+              ok = ptx::mbar_wait_bounded_fast<20>(tmem_empty_bar(buf), buf_phase ^ 1u, abort_flag, 4, WAIT_BUDGET_NS);
+              if (!ok) break;
+              ptx::tc_fence_after_sync();
+              const uint32_t d = tmem_base + (uint32_t)(buf * BN);
+              if (part == 0) {                           // the small products, the smallest first
+                mma(d, al + AP, bl + 2 * BP, 0u);        // mid * lo
+                mma(d, al + 2 * AP, bl + BP, 1u);        // lo * mid
+                mma(d, al, bl + 2 * BP, 1u);             // hi * lo
+                mma(d, al + 2 * AP, bl, 1u);             // lo * hi
+                mma(d, al + AP, bl + BP, 1u);            // mid * mid
+                mma(d, al, bl + BP, 1u);                 // hi * mid
+                mma(d, al + AP, bl, 1u);                 // mid * hi
+              } else {
+                mma(d, al, bl, 0u);                      // hi * hi
+                commit(empty_b(sb));
+                if (t == share - 1) commit(empty_a(sa));
+              }
+              commit(tmem_full_bar(buf));
+              if (++buf == L::BUFS) {
+                buf = 0;
+                buf_phase ^= 1u;
+              }
+            }
             if (++sb == L::B_STAGES) {
               sb = 0;
               pb ^= 1u;
-            }
-            if (++buf == L::BUFS) {
-              buf = 0;
-              buf_phase ^= 1u;
             }
           }
           if (++sa == A_STAGES) {
@@ -389,8 +402,8 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       float acc[L::EPI_COLS];
 #pragma unroll
       for (int j = 0; j < L::EPI_COLS; ++j) acc[j] = 0.f;
-      const int chunks = (u1 - u0) * share;
-      for (int q = 0; q < chunks && ok; ++q) {
+      const int sums = (u1 - u0) * share * PARTS;
+      for (int q = 0; q < sums && ok; ++q) {
         ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded_fast<20>(tmem_full_bar(buf), buf_phase, abort_flag, 6, WAIT_BUDGET_NS));
         if (!ok) break;
         ptx::tc_fence_after_sync();
@@ -417,7 +430,6 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       const int ncols = min(L::EPI_COLS, p.oc - co0);
       float* const out0 = args.y + (partial ? split * args.plane : 0) + ((long long)img * p.oc + co0) * ohow + h * p.ow + w;
       const bool relu = !partial && p.do_relu;
-      const float gain = partial ? 0.f : TRUNCATION;   // (partial sums: once, when they are added up)
       const float ceiling = p.relu_limit > 0.f ? p.relu_limit : INFINITY;
       uint32_t again[L::EPI_COLS / 32];           // results to recompute (a plain zero needs no second look)
       float* o = out0;
@@ -428,7 +440,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         for (int j = 0; j < 32; ++j) {
           const float s = acc[i * 32 + j], m = fabsf(s);
           if (!(m <= 3.402823466e38f && (m >= 8.67e-19f || m == 0.f))) again[i] |= 1u << j;
-          const float v = s + fmaf(s, gain, __shfl_sync(0xffffffffu, bias[i], j));
+          const float v = s + __shfl_sync(0xffffffffu, bias[i], j);
           if (valid && i * 32 + j < ncols) *o = relu ? fminf(fmaxf(v, 0.f), ceiling) : v;
           o += ohow;
           asm volatile("" : "+l"(o));   // one running address: 64 of them kept ahead spilled the sums
@@ -493,7 +505,7 @@ struct UmmaChoice {
 };
 
 // Tile form and K splits of a launch over `images` images, by a model in nanoseconds.  A chunk costs what its operands cost
-// to bring in (75 bytes per ns and SM, measured) or its 24 MMAs, whichever is more.  These read both operands from shared
+// to bring in (75 bytes per ns and SM, measured) or its 32 MMAs, whichever is more.  These read both operands from shared
 // memory, which sets their pace (128 bytes per clock: 62 clocks measured at 256 x 128 x 16 where the tensor pipe needs 32), so
 // that 256 channels cost little more than 128.  A round of tiles costs its chunks, or its stores, plus 1.5 us for the
 // pipeline's start; partial sums cost a launch and a pass over the output's planes.
@@ -512,7 +524,7 @@ UmmaChoice choose(const TopConvPlan& p, int images, int sms) {
     const int tile_m = pair ? 2 * TILE_M : TILE_M;
     const int m_tiles = (int)((rows + tile_m - 1) / tile_m), n_tiles = (p.oc + bn - 1) / bn;
     const double bytes = 3.0 * CHUNK_BYTES * ((double)TILE_M / best.share + (pair ? bn / 2 : bn));
-    const double mma = bn == 64 ? 600 : (bn == 128 ? 800 : 1100), chunk = bytes / 75.0 > mma ? bytes / 75.0 : mma;
+    const double mma = bn == 64 ? 800 : (bn == 128 ? 1070 : 1470), chunk = bytes / 75.0 > mma ? bytes / 75.0 : mma;
     const double store = TILE_M * bn * 4.0 / 20.0;
     for (int sp = 1; sp <= 8 && sp <= best.units; ++sp) {
       const long long tiles = (long long)m_tiles * n_tiles * sp, slots = pair ? sms / 2 : sms;
@@ -652,7 +664,7 @@ int top_conv_umma_launch(const TopConvPlan& plan, const float* x, const float* w
     else if (c.bn == 128) B200Q_TRY((launch_umma<128, true>(ta, tb, a, sms, s)));
     else B200Q_TRY((launch_umma<256, true>(ta, tb, a, sms, s)));
     if (a.splits > 1)
-      B200Q_TRY(top_conv_reduce_launch(partial, bias, yg, a.plane, a.splits, p.oc, p.oh * p.ow, p.do_relu, p.relu_limit, TRUNCATION, s));
+      B200Q_TRY(top_conv_reduce_launch(partial, bias, yg, a.plane, a.splits, p.oc, p.oh * p.ow, p.do_relu, p.relu_limit, s));
   }
   return B200Q_OK;
 }
