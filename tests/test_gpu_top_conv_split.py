@@ -133,6 +133,26 @@ def test_values_outside_the_split(value):
     assert bool(((got - ref).abs()[fin] <= (mag * 2.0**-20)[fin] + ref.abs()[fin] * 2.0**-23).all())
 
 
+@pytest.mark.parametrize("case", [CASES[i] for i in (0, 2, 4, 6, 9)])
+@pytest.mark.parametrize("xs,ws", [(1e-36, 1e20), (1e-41, 1e20), (1e20, 1e-36), (1e-20, 1e-22), (1e-30, 1.0), (1.0, 1e-38)])
+@pytest.mark.parametrize("part", [False, True])
+def test_operands_near_underflow(case, xs, ws, part):
+    """Small operands whose low parts underflow although the results do not, results that are subnormal, zeros that underflow made;
+    everywhere, or in one image row and one channel only.  Beyond the bound of normal values, a product of fp32 FMAs is rounded to
+    multiples of 2^-149, twice that allowed here."""
+    n, ic, ih, iw, oc, kh, kw, stride, pads, dil = case
+    x, w, _ = draw(13, n, ic, ih, iw, oc, kh, kw)
+    if part:
+        x[0, :, ih // 2] *= xs
+        w[oc // 3] *= ws
+    else:
+        x, w = x * xs, w * ws
+    got = Conv(w, None, ih, iw, stride, pads, dil)(x)
+    ref = ref64(x, w, None, stride, pads, dil)
+    mag = ref64(x.abs(), w.abs(), None, stride, pads, dil)
+    assert bool(((got.double() - ref).abs() <= mag * 2.0**-21 + ref.abs() * 2.0**-23 + ic * kh * kw * 2.0**-148).all())
+
+
 def test_capture_and_two_streams():
     x, w, b = draw(9, 6, 64, 28, 28, 128, 3, 3)
     conv = Conv(w, b, 28, 28, 1, (1, 1, 1, 1))

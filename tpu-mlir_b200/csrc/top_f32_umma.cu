@@ -23,8 +23,9 @@
 //                      and chunk carries the three planes), warp 1 issues the MMAs, the others add up and store NCHW fp32.
 // Images are taken a group at a time so that the planes stay in the L2 between the two kernels.
 //
-// Infinities, NaN, sums that overflow and results so small that the low planes may have underflowed are recomputed by a plain
-// FMA loop over the fp32 operands: such results are what the CUDA-core kernel gives.
+// Three things are recomputed by a plain FMA loop over the fp32 operands, which gives what the CUDA-core kernel gives: infinities
+// and NaN, sums that overflow, and results that underflow may have touched.  The last is decided from the operands: the split
+// kernels note the smallest and largest exponents of every 32 rows and of every channel (see `may_be_lost`).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -68,17 +69,45 @@ struct UmmaLayout {
 };
 
 // x = h + m + l, h rounded to nearest to 6 significant bits, m and l to bf16's 8: 18 bits are left for m, 9 of them and a sign
-// (or 2^8) for l.  Exact for every float whose low part is not subnormal.
+// (or 2^8) for l.  Exact for every float whose low part is not subnormal.  (An infinity and a NaN leave a NaN in m, and values
+// that round to an infinite h do too: their sums are recomputed.)
 __device__ __forceinline__ void split3(float x, uint16_t& h, uint16_t& m, uint16_t& l) {
-  const uint32_t u = __float_as_uint(x);
-  const __nv_bfloat16 bh = (u & 0x7f800000u) == 0x7f800000u ? __float2bfloat16_rn(x)
-                                                            : __ushort_as_bfloat16((unsigned short)(((u + 0x20000u) & 0xfffc0000u) >> 16));
-  const float r1 = x - __bfloat162float(bh);
+  const uint32_t hb = (__float_as_uint(x) + 0x20000u) & 0xfffc0000u;
+  const float r1 = x - __uint_as_float(hb);
   const __nv_bfloat16 bm = __float2bfloat16_rn(r1);
   const float r2 = r1 - __bfloat162float(bm);
-  h = __bfloat16_as_ushort(bh);
+  h = (uint16_t)(hb >> 16);
   m = __bfloat16_as_ushort(bm);
   l = __bfloat16_as_ushort(__float2bfloat16_rn(r2));
+}
+
+// Exponents (biased) of a set of values: largest << 16 | smallest of the non-zero ones.
+constexpr uint32_t NO_VALUE = 511;             // "smallest" of a set of zeros
+constexpr int RANGE_ROWS = 32;                 // rows that share a range
+
+// (a NaN is left out: what it touches is NaN and recomputed for that)
+__device__ __forceinline__ void range_add(float v, float& largest, uint32_t& smallest) {
+  largest = fmaxf(largest, fabsf(v));
+  smallest = min(smallest, __float_as_uint(v) * 2u - 1u);   // drops the sign; zero wraps round to the largest number
+}
+__device__ __forceinline__ uint32_t range_pack(float largest, uint32_t smallest) {   // over the warp
+  const uint32_t l = __reduce_max_sync(0xffffffffu, __float_as_uint(largest));
+  smallest = __reduce_min_sync(0xffffffffu, smallest);
+  return ((l >> 23) << 16) | (smallest == 0xffffffffu ? NO_VALUE : (smallest + 1u) >> 24);
+}
+__device__ __forceinline__ uint32_t range_join(uint32_t a, uint32_t b) {
+  return max(a & 0xffff0000u, b & 0xffff0000u) | min(a & 0xffffu, b & 0xffffu);
+}
+
+// A sum of `k` products from operands of the given ranges: 0 if underflow cannot have touched it, else the magnitude from
+// which on it does not matter.  Nothing is lost while every part is a normal bf16 (the lowest bit of an operand is 2^-23 of its
+// leading one: exponents from -102) and every product of operands is at least 2^-90 (what its smallest parts lose is below
+// 2^-33 of it).  Otherwise a product can lose 3 * 2^-126 of either operand and eight parts of 2^-126: the sum is off by at most
+// k * 2^-124 * (max|x| + max|w| + 2), which is 2^-26 of a result of this size, a quarter of an fp32 rounding.
+__device__ __forceinline__ float may_be_lost(uint32_t x, uint32_t w, float k) {
+  const uint32_t xs = x & 0xffffu, ws = w & 0xffffu;
+  if (xs == NO_VALUE || ws == NO_VALUE || (xs >= 25u && ws >= 25u && xs + ws >= 164u)) return 0.f;
+  return k * 0x1p-98f * (ldexpf(1.f, (int)(x >> 16) - 126) + ldexpf(1.f, (int)(w >> 16) - 126) + 2.f);
 }
 
 struct SplitArgs {
@@ -88,12 +117,14 @@ struct SplitArgs {
   int cp;                  // channels per tap, rounded up to 8
   long long rows;          // images x rh x rw
   long long pitch;         // elements per row: taps (of this form) x cp
+  uint32_t* range;         // [tap][64 channels][32 rows]
 };
 
 // One block: 32 rows x 64 channels of one tap.  Memory bound (4 bytes read, 6 written per element): a warp reads 32
 // neighbouring pixels of eight channels, the block turns them in shared memory and writes 128-byte channel runs.
 __global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, const SplitArgs a) {
   __shared__ __align__(16) uint16_t tile[3][32][CHUNK + 8];
+  __shared__ uint32_t ranges[8];
   ptx::griddep_launch_dependents();   // the second kernel may set itself up meanwhile; it waits for this one's end
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = blockIdx.y * CHUNK + warp * 8;
@@ -115,6 +146,12 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict_
         if (c0 + i < a.ic) v[i] = __ldg(src + (long long)i * hw);
     }
   }
+  float largest = 0.f;
+  uint32_t smallest = 0xffffffffu;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) range_add(v[i], largest, smallest);
+  const uint32_t range = range_pack(largest, smallest);
+  if (lane == 0) ranges[warp] = range;
   uint32_t p[3][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -129,6 +166,12 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict_
   for (int q = 0; q < 3; ++q)
     *reinterpret_cast<uint4*>(&tile[q][lane][warp * 8]) = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
   __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t all = ranges[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) all = range_join(all, ranges[i]);
+    a.range[((long long)tap * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = all;
+  }
   const int rr = threadIdx.x >> 3, piece = (threadIdx.x & 7) * 8;
   const long long orow = (long long)blockIdx.x * 32 + rr;
   const int c = blockIdx.y * CHUNK + piece;
@@ -155,6 +198,19 @@ __global__ void split_weight_kernel(const float* __restrict__ w, __nv_bfloat16* 
   out[2 * total + i] = __ushort_as_bfloat16(l);
 }
 
+// Exponents of every output channel's weights, once per handle: one block per channel
+__global__ void __launch_bounds__(128) weight_range_kernel(const float* __restrict__ w, uint32_t* __restrict__ range, long long per_channel) {
+  __shared__ uint32_t ranges[4];
+  const float* src = w + blockIdx.x * per_channel;
+  float largest = 0.f;
+  uint32_t smallest = 0xffffffffu;
+  for (long long i = threadIdx.x; i < per_channel; i += 128) range_add(src[i], largest, smallest);
+  const uint32_t r = range_pack(largest, smallest);
+  if ((threadIdx.x & 31) == 0) ranges[threadIdx.x >> 5] = r;
+  __syncthreads();
+  if (threadIdx.x == 0) range[blockIdx.x] = range_join(range_join(ranges[0], ranges[1]), range_join(ranges[2], ranges[3]));
+}
+
 struct UmmaArgs {
   TopConvPlan p;             // n: the images of this launch
   // k is walked in units of (tap group, 64 channels); a unit is `share` chunks, the taps of one filter row on one load of A
@@ -171,6 +227,10 @@ struct UmmaArgs {
   const float* bias;
   float* y;                  // splits > 1: planes of partial sums
   long long plane;           // floats of one plane
+  const uint32_t* x_range;   // [x_groups][x_blocks], x_blocks of 32 rows each
+  const uint32_t* w_range;   // [oc]
+  float k_total;             // products of one output
+  int x_blocks, x_groups, halo;   // halo: rows past a tile's last that its last row's taps reach
 };
 
 // The sum of units [u0, u1) for one output by fp32 FMAs
@@ -399,6 +459,19 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 #pragma unroll
       for (int i = 0; i < L::EPI_COLS / 32; ++i)
         bias[i] = (args.bias && !partial && co0 + i * 32 + lane < p.oc) ? __ldg(args.bias + co0 + i * 32 + lane) : 0.f;
+      // ranges of the rows this warp's taps read (lane by lane) and of its channels; first looked at after the sums
+      uint32_t x_range = NO_VALUE, w_range[L::EPI_COLS / 32];
+      {
+        const int row0 = min(row - lane, args.rows - 1), b0 = row0 / RANGE_ROWS;
+        const int nb = min(row0 + 31 + args.halo, args.rows - 1) / RANGE_ROWS - b0 + 1;
+        for (int i = lane; i < nb * args.x_groups; i += 32) {
+          const int gr = i / nb;
+          const uint32_t v = __ldcg(args.x_range + (long long)gr * args.x_blocks + b0 + (i - gr * nb));
+          x_range = i < 32 ? v : range_join(x_range, v);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < L::EPI_COLS / 32; ++i) w_range[i] = co0 + i * 32 + lane < p.oc ? __ldg(args.w_range + co0 + i * 32 + lane) : NO_VALUE;
       float acc[L::EPI_COLS];
 #pragma unroll
       for (int j = 0; j < L::EPI_COLS; ++j) acc[j] = 0.f;
@@ -431,15 +504,26 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       float* const out0 = args.y + (partial ? split * args.plane : 0) + ((long long)img * p.oc + co0) * ohow + h * p.ow + w;
       const bool relu = !partial && p.do_relu;
       const float ceiling = p.relu_limit > 0.f ? p.relu_limit : INFINITY;
-      uint32_t again[L::EPI_COLS / 32];           // results to recompute (a plain zero needs no second look)
+      x_range = (__reduce_max_sync(0xffffffffu, x_range >> 16) << 16) | __reduce_min_sync(0xffffffffu, x_range & 0xffffu);
+      uint32_t again[L::EPI_COLS / 32];           // results to recompute
       float* o = out0;
 #pragma unroll
       for (int i = 0; i < L::EPI_COLS / 32; ++i) {
         again[i] = 0u;
+        const float lost = may_be_lost(x_range, w_range[i], args.k_total);   // lane j: channel j's
+        if (__any_sync(0xffffffffu, lost > 0.f)) {
+          for (int j = 0; j < 32; ++j) {
+            const float from = __shfl_sync(0xffffffffu, lost, j);
+            float s = 0.f;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) s = q == j ? acc[i * 32 + q] : s;   // (rare: no indexing of registers)
+            if (fabsf(s) < from) again[i] |= 1u << j;
+          }
+        }
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const float s = acc[i * 32 + j], m = fabsf(s);
-          if (!(m <= 3.402823466e38f && (m >= 8.67e-19f || m == 0.f))) again[i] |= 1u << j;
+          const float s = acc[i * 32 + j];
+          if (!(fabsf(s) <= 3.402823466e38f)) again[i] |= 1u << j;
           const float v = s + __shfl_sync(0xffffffffu, bias[i], j);
           if (valid && i * 32 + j < ncols) *o = relu ? fminf(fmaxf(v, 0.f), ceiling) : v;
           o += ohow;
@@ -485,6 +569,18 @@ size_t image_bytes(const TopConvPlan& p) {
   const size_t taps = (size_t)p.kh * p.kw, cp = cp_of(p);
   if (shifted_rows(p)) return 6 * cp * (size_t)(p.oh + (p.kh - 1) * p.dh) * (p.ow + (p.kw - 1) * p.dw);
   return 6 * cp * taps * (size_t)p.oh * p.ow;
+}
+
+size_t image_rows(const TopConvPlan& p) {
+  return shifted_rows(p) ? (size_t)(p.oh + (p.kh - 1) * p.dh) * (p.ow + (p.kw - 1) * p.dw) : (size_t)p.oh * p.ow;
+}
+
+size_t scratch_plane_bytes(const TopConvPlan& p, int images) { return ((size_t)images * image_bytes(p) + 1023) & ~(size_t)1023; }
+
+size_t scratch_range_bytes(const TopConvPlan& p, int images) {
+  const size_t blocks = (images * image_rows(p) + RANGE_ROWS - 1) / RANGE_ROWS;
+  const size_t groups = (size_t)((cp_of(p) + CHUNK - 1) / CHUNK) * (shifted_rows(p) ? 1 : p.kh * p.kw);
+  return (blocks * groups * sizeof(uint32_t) + 1023) & ~(size_t)1023;
 }
 
 // Planes of one group of images: half of the L2, so that the second kernel finds what the first one wrote
@@ -571,7 +667,9 @@ int launch_umma(const CUtensorMap& ta, const CUtensorMap& tb, const UmmaArgs& a,
 
 }  // namespace
 
-size_t top_conv_umma_weight_bytes(const TopConvPlan& p) { return (size_t)3 * 2 * p.oc * p.kh * p.kw * cp_of(p); }
+// the planes, then the channels' ranges
+size_t weight_plane_bytes(const TopConvPlan& p) { return ((size_t)3 * 2 * p.oc * p.kh * p.kw * cp_of(p) + 255) & ~(size_t)255; }
+size_t top_conv_umma_weight_bytes(const TopConvPlan& p) { return weight_plane_bytes(p) + (size_t)p.oc * sizeof(uint32_t); }
 
 bool top_conv_umma_takes(const TopConvPlan& p) {
   if (p.groups != 1 || p.ic < 32 || p.oc < 32) return false;
@@ -587,14 +685,18 @@ int top_conv_umma_prepare(const TopConvPlan& p, const float* w_oihw, void* plane
   const long long total = (long long)p.oc * taps * cp;
   split_weight_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(w_oihw, static_cast<__nv_bfloat16*>(planes), p.oc, p.ic, taps, cp);
   CUDA_TRY(cudaGetLastError());
+  weight_range_kernel<<<(unsigned)p.oc, 128, 0, s>>>(w_oihw, reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(planes) + weight_plane_bytes(p)),
+                                                     (long long)p.ic * taps);
+  CUDA_TRY(cudaGetLastError());
   return B200Q_OK;
 }
 
-// The scratch a call needs: the planes of one group of images, then the partial sums of one group (if it splits K).
+// The scratch a call needs: the planes of one group of images and their ranges, then the partial sums of one group (if it
+// splits K).
 size_t top_conv_umma_scratch(const TopConvPlan& p, int sms) {
   const int g = group_images(p);
   const UmmaChoice c = choose(p, g, sms);
-  size_t need = ((size_t)g * image_bytes(p) + 1023) & ~(size_t)1023;
+  size_t need = scratch_plane_bytes(p, g) + scratch_range_bytes(p, g);
   if (c.splits > 1) need += (size_t)c.splits * g * p.oc * p.oh * p.ow * 4;
   return need;
 }
@@ -604,8 +706,9 @@ int top_conv_umma_launch(const TopConvPlan& plan, const float* x, const float* w
   const int g = group_images(plan), cp = cp_of(plan), taps = plan.kh * plan.kw;
   const bool shifted = shifted_rows(plan);
   const UmmaChoice c = choose(plan, g, sms);
-  const size_t plane_bytes = ((size_t)g * image_bytes(plan) + 1023) & ~(size_t)1023;
-  float* partial = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + plane_bytes);
+  const size_t plane_bytes = scratch_plane_bytes(plan, g);
+  uint32_t* const range = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(scratch) + plane_bytes);
+  float* partial = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + plane_bytes + scratch_range_bytes(plan, g));
   for (int i0 = 0; i0 < plan.n; i0 += g) {
     TopConvPlan p = plan;
     p.n = plan.n - i0 < g ? plan.n - i0 : g;
@@ -620,7 +723,8 @@ int top_conv_umma_launch(const TopConvPlan& plan, const float* x, const float* w
       sa.rh = p.oh; sa.rw = p.ow; sa.sh = p.sh; sa.sw = p.sw; sa.pitch = (long long)taps * cp;
     }
     sa.rows = (long long)p.n * sa.rh * sa.rw;
-    dim3 grid((unsigned)((sa.rows + 31) / 32), (unsigned)((cp + CHUNK - 1) / CHUNK), (unsigned)(shifted ? 1 : taps));
+    sa.range = range;
+    dim3 grid((unsigned)((sa.rows + RANGE_ROWS - 1) / RANGE_ROWS), (unsigned)((cp + CHUNK - 1) / CHUNK), (unsigned)(shifted ? 1 : taps));
     split_f32_kernel<<<grid, 256, 0, s>>>(xg, static_cast<__nv_bfloat16*>(scratch), sa);
     CUDA_TRY(cudaGetLastError());
 
@@ -644,6 +748,12 @@ int top_conv_umma_launch(const TopConvPlan& plan, const float* x, const float* w
     a.x = xg; a.wt = wt; a.bias = bias;
     a.plane = (long long)p.n * p.oc * p.oh * p.ow;
     a.y = a.splits > 1 ? partial : yg;
+    a.x_range = range;
+    a.w_range = reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(w_planes) + weight_plane_bytes(p));
+    a.x_blocks = (int)grid.x;
+    a.x_groups = (int)(grid.y * grid.z);
+    a.halo = shifted ? (p.kh - 1) * a.tap_h + (p.kw - 1) * a.tap_w : 0;
+    a.k_total = (float)taps * (float)p.ic;
 
     CUtensorMap ta, tb;
     {
