@@ -133,6 +133,18 @@ def test_values_outside_the_split(value):
     assert bool(((got - ref).abs()[fin] <= (mag * 2.0**-20)[fin] + ref.abs()[fin] * 2.0**-23).all())
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("stride", [1, 2])
+def test_weights_that_are_not_finite_meet_the_border(value, stride):
+    """The border counts as zeros: an infinite weight on it gives NaN, as it does in a sum over the padded image."""
+    x, w, b = draw(3, 2, 64, 9, 9, 96, 3, 3)
+    w[5, 3, 0, 2] = value
+    got = Conv(w, b, 9, 9, stride, (1, 1, 1, 1))(x)
+    ref = ref64(x, w, b, stride, (1, 1, 1, 1), 1).float()
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(got[torch.isinf(ref)], ref[torch.isinf(ref)])
+    assert bool(torch.isnan(ref[:, 5, 0]).all())
+
+
 @pytest.mark.parametrize("case", [CASES[i] for i in (0, 2, 4, 6, 9)])
 @pytest.mark.parametrize("xs,ws", [(1e-36, 1e20), (1e-41, 1e20), (1e20, 1e-36), (1e-20, 1e-22), (1e-30, 1.0), (1.0, 1e-38)])
 @pytest.mark.parametrize("part", [False, True])

@@ -250,8 +250,9 @@ __device__ __noinline__ float conv_sum_plain(const UmmaArgs& a, int img, int h, 
         if (tap >= taps || c >= p.ic) continue;
         const int fy = tap / p.kw, fx = tap - fy * p.kw;
         const int ih = h * p.sh + fy * p.dh - p.pht, iw = w * p.sw + fx * p.dw - p.pwl;
-        if ((unsigned)ih >= (unsigned)p.ih || (unsigned)iw >= (unsigned)p.iw) continue;
-        s = fmaf(__ldg(a.wt + ((long long)c * taps + tap) * p.oc + co), __ldg(a.x + (((long long)img * p.ic + c) * p.ih + ih) * p.iw + iw), s);
+        const bool inside = (unsigned)ih < (unsigned)p.ih && (unsigned)iw < (unsigned)p.iw;   // the border is zeros: 0 * inf is NaN
+        const float xv = inside ? __ldg(a.x + (((long long)img * p.ic + c) * p.ih + ih) * p.iw + iw) : 0.f;
+        s = fmaf(__ldg(a.wt + ((long long)c * taps + tap) * p.oc + co), xv, s);
       }
     }
   }
