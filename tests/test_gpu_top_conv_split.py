@@ -165,6 +165,31 @@ def test_operands_near_underflow(case, xs, ws, part):
     assert bool(((got.double() - ref).abs() <= mag * 2.0**-21 + ref.abs() * 2.0**-23 + ic * kh * kw * 2.0**-148).all())
 
 
+def test_time_does_not_hang_on_the_values():
+    """Dead channels (weights near zero, biases that swallow what they give) cost nothing, an infinity or a tensor of NaN a bounded
+    number of recomputed sums.  (Without the bias in the decision: 15 times; one sum after the other: 400 times.)"""
+    x, w, b = draw(2, 32, 256, 14, 14, 256, 3, 3)
+
+    def time_of(x, w):
+        conv = Conv(w, b, 14, 14, 1, (1, 1, 1, 1))
+        conv(x)
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(8)]
+        for e in ev:
+            e.record()
+            conv(x)
+        torch.cuda.synchronize()
+        return min(a.elapsed_time(z) for a, z in zip(ev, ev[1:]))
+    plain = time_of(x, w)
+    for scale in (1e-20, 1e-38):
+        dead = w.clone()
+        dead[::32] *= scale
+        assert time_of(x, dead) < 3 * plain
+    one = x.clone()
+    one[0, 0, 5, 5] = float("inf")
+    assert time_of(one, w) < 100 * plain
+    assert time_of(x * float("nan"), w) < 100 * plain
+
+
 def test_capture_and_two_streams():
     x, w, b = draw(9, 6, 64, 28, 28, 128, 3, 3)
     conv = Conv(w, b, 28, 28, 1, (1, 1, 1, 1))

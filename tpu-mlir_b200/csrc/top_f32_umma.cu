@@ -233,30 +233,70 @@ struct UmmaArgs {
   int x_blocks, x_groups, halo;   // halo: rows past a tile's last that its last row's taps reach
 };
 
-// The sum of units [u0, u1) for one output by fp32 FMAs
-__device__ __noinline__ float conv_sum_plain(const UmmaArgs& a, int img, int h, int w, int co, int u0, int u1) {
-  const TopConvPlan& p = a.p;
-  const int taps = p.kh * p.kw;
-  float s = 0.f;
+// Units [u0, u1) of k as runs of channels of one tap: f(tap, first channel, end), until it returns false
+template <typename F>
+__device__ __forceinline__ void for_runs(const UmmaArgs& a, int u0, int u1, F f) {
+  const int taps = a.p.kh * a.p.kw;
   for (int u = u0; u < u1; ++u) {
-    const int group = u / a.units_per_tap, kc = u - group * a.units_per_tap;
-    for (int t = 0; t < a.share; ++t) {
-      for (int e = 0; e < CHUNK; ++e) {
-        int tap = group * a.share + t, c = kc * CHUNK + e;
-        if (a.one_row) {
-          tap = c / a.cp;
-          c -= tap * a.cp;
-        }
-        if (tap >= taps || c >= p.ic) continue;
-        const int fy = tap / p.kw, fx = tap - fy * p.kw;
-        const int ih = h * p.sh + fy * p.dh - p.pht, iw = w * p.sw + fx * p.dw - p.pwl;
-        const bool inside = (unsigned)ih < (unsigned)p.ih && (unsigned)iw < (unsigned)p.iw;   // the border is zeros: 0 * inf is NaN
-        const float xv = inside ? __ldg(a.x + (((long long)img * p.ic + c) * p.ih + ih) * p.iw + iw) : 0.f;
-        s = fmaf(__ldg(a.wt + ((long long)c * taps + tap) * p.oc + co), xv, s);
+    const int group = u / a.units_per_tap, e0 = (u - group * a.units_per_tap) * CHUNK;
+    if (!a.one_row) {
+      for (int tap = group * a.share; tap < min(taps, (group + 1) * a.share); ++tap)
+        if (e0 < a.p.ic && !f(tap, e0, min(e0 + CHUNK, a.p.ic))) return;
+    } else {
+      const int end = min(e0 + CHUNK, taps * a.cp);
+      for (int e = e0; e < end;) {
+        const int tap = e / a.cp, c = e - tap * a.cp, n = min(end - e, a.cp - c);
+        if (c < a.p.ic && !f(tap, c, min(c + n, a.p.ic))) return;
+        e += n;
       }
     }
   }
-  return s;
+}
+
+// Results of a warp's rows (`row` is this lane's) in 32 channels from `co` on, by fp32 FMAs: `again` has this lane's.  Four channels at a time from one value of x, so that a layer full of infinities costs a few times what the
+// CUDA-core kernel takes for it; a group of four leaves off when nothing but NaN is left.
+__device__ __noinline__ void recompute(const UmmaArgs& a, int row, int co, int split, uint32_t again) {
+  const TopConvPlan& p = a.p;
+  const int per = a.rh * a.rw, img = row / per, rem = row - img * per, h = rem / a.rw, w = rem - h * a.rw;
+  const bool valid = row < a.rows && h < p.oh && w < p.ow;
+  const long long hw = (long long)p.ih * p.iw, w_step = (long long)p.kh * p.kw * p.oc;
+  const int u0 = split * a.units_per_split, u1 = min(a.units, u0 + a.units_per_split);
+  const bool partial = a.splits > 1;
+  float* const out = a.y + (partial ? split * a.plane : 0) + ((long long)img * p.oc + co) * p.oh * p.ow + h * p.ow + w;
+  const float ceiling = p.relu_limit > 0.f ? p.relu_limit : INFINITY;
+  if (!valid) again = 0u;
+  if (p.oc - co < 32) again &= (1u << max(p.oc - co, 0)) - 1u;
+  uint32_t columns = __reduce_or_sync(0xffffffffu, again);
+  while (columns != 0u) {
+    int col[4];   // the next four channels (the last one again where fewer are left)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      col[q] = columns != 0u ? __ffs((int)columns) - 1 : col[q > 0 ? q - 1 : 0];
+      columns &= columns - 1u;
+    }
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for_runs(a, u0, u1, [&](int tap, int c0, int c1) {
+      const int fy = tap / p.kw, fx = tap - fy * p.kw;
+      const int y = h * p.sh + fy * p.dh - p.pht, x = w * p.sw + fx * p.dw - p.pwl;
+      const bool inside = valid && (unsigned)y < (unsigned)p.ih && (unsigned)x < (unsigned)p.iw;   // the border is zeros: 0 * inf is NaN
+      const float* xp = a.x + (inside ? (((long long)img * p.ic + c0) * p.ih + y) * p.iw + x : 0);
+      const float* wp = a.wt + c0 * w_step + (long long)tap * p.oc + co;
+#pragma unroll 4
+      for (int c = c0; c < c1; ++c, wp += w_step) {
+        const float xv = inside ? __ldg(xp) : 0.f;
+        if (inside) xp += hw;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] = fmaf(__ldg(wp + col[q]), xv, s[q]);
+      }
+      return !__all_sync(0xffffffffu, !valid || (s[0] != s[0] && s[1] != s[1] && s[2] != s[2] && s[3] != s[3]));
+    });
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float v = s[q] + (a.bias && !partial ? __ldg(a.bias + co + col[q]) : 0.f);
+      if (!partial && p.do_relu) v = fminf(fmaxf(v, 0.f), ceiling);
+      if ((again >> col[q]) & 1u) out[(long long)col[q] * p.oh * p.ow] = v;
+    }
+  }
 }
 
 template <int BN, bool PAIR>
@@ -459,7 +499,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       float bias[L::EPI_COLS / 32];               // lane j holds channel j's; handed round when the results are stored
 #pragma unroll
       for (int i = 0; i < L::EPI_COLS / 32; ++i)
-        bias[i] = (args.bias && !partial && co0 + i * 32 + lane < p.oc) ? __ldg(args.bias + co0 + i * 32 + lane) : 0.f;
+        bias[i] = (args.bias && co0 + i * 32 + lane < p.oc) ? __ldg(args.bias + co0 + i * 32 + lane) : 0.f;
       // ranges of the rows this warp's taps read (lane by lane) and of its channels; first looked at after the sums
       uint32_t x_range = NO_VALUE, w_range[L::EPI_COLS / 32];
       {
@@ -511,7 +551,9 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 #pragma unroll
       for (int i = 0; i < L::EPI_COLS / 32; ++i) {
         again[i] = 0u;
-        const float lost = may_be_lost(x_range, w_range[i], args.k_total);   // lane j: channel j's
+        float lost = may_be_lost(x_range, w_range[i], args.k_total);   // lane j: channel j's
+        if (fabsf(bias[i]) >= lost) lost = 0.f;     // the bias swallows it (a dead channel: weights near zero, any bias)
+        if (partial) bias[i] = 0.f;                 // added with the partial sums
         if (__any_sync(0xffffffffu, lost > 0.f)) {
           for (int j = 0; j < 32; ++j) {
             const float from = __shfl_sync(0xffffffffu, lost, j);
@@ -534,18 +576,10 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       // the rare ones, and everything if a wait ran out (the sums are lost, and say so)
 #pragma unroll
       for (int i = 0; i < L::EPI_COLS / 32; ++i) {
-        if (!ok) again[i] = 0xffffffffu;
-        const bool any = __any_sync(0xffffffffu, valid && again[i] != 0u);
-        if (!any) continue;
-        for (int j = 0; j < 32; ++j) {
-          const float b = __shfl_sync(0xffffffffu, bias[i], j);
-          if (!valid || i * 32 + j >= ncols || !((again[i] >> j) & 1u)) continue;
-          float v = __int_as_float(0x7fffffff);
-          if (ok) {
-            v = conv_sum_plain(args, img, h, w, co0 + i * 32 + j, u0, u1) + b;
-            if (relu) v = fminf(fmaxf(v, 0.f), ceiling);
-          }
-          out0[(long long)(i * 32 + j) * ohow] = v;
+        if (!ok) {
+          for (int j = i * 32; valid && j < min(i * 32 + 32, ncols); ++j) out0[(long long)j * ohow] = __int_as_float(0x7fffffff);
+        } else if (__any_sync(0xffffffffu, valid && again[i] != 0u)) {
+          recompute(args, row, co0 + i * 32, split, again[i]);
         }
       }
     }
