@@ -373,7 +373,7 @@ int b200q_a16_w4_dev_dt(const void *x, const void *wq, const void *scale, const 
                         void *y, int64_t M, int64_t N, int64_t K, int32_t group, int32_t dtype, int32_t *status,
                         void *stream);
 
-/* Test aid (no counterpart in the reference): makes a bounded wait of the tensor-core INT8 GEMM/convolution kernel run
+/* Test aid (no counterpart in the reference): makes a bounded wait of the tensor-core GEMM/convolution kernels run
  * out without faulting anything.  While extra_tx_bytes > 0 every pipeline stage's barrier expects that many bytes more
  * than the stage's loads deliver, so the consumer's wait ends after `budget_ns` (0 = the default of 2 s) with the
  * kernel's status set to the wait site; the calls then return B200Q_ERR_TIMEOUT and leave the context usable.
@@ -502,6 +502,10 @@ int b200q_top_conv2d_inference(const b200q_top_conv_desc *desc, float *const *in
 /* Device face: the handle keeps a transposed copy of the filter; `bias` stays the caller's.  run() takes any batch. */
 int b200q_top_conv2d_dev_create(const b200q_top_conv_desc *desc, const float *filter_oihw, const float *bias, void **handle);
 int b200q_top_conv2d_dev_run(void *handle, const float *x, float *y, int64_t batch, void *stream);
+/* Synchronises the stream and reports a kernel-side timeout, if any: the output is not valid then.  set_status names a device
+ * word of the caller's for it instead (0 beforehand; NULL: the handle's own), so that one read serves many handles. */
+int b200q_top_conv2d_dev_status(void *handle, void *stream);
+int b200q_top_conv2d_dev_set_status(void *handle, int32_t *status);
 void b200q_top_conv2d_dev_output_shape(void *handle, int64_t *oh, int64_t *ow);
 void b200q_top_conv2d_dev_destroy(void **handle);
 /* top::MatMulOp without transposes: y[M,N] = relu(x[M,K] * w[K,N] + bias[N]) (lib/Dialect/Top/Interfaces/MatMul.cpp). */

@@ -142,6 +142,53 @@ def test_sharded_calibrator_two_ranks_matches_streaming_reference(tmp_path, monk
         merge_shards([str(tmp_path / "shard0.npz")], math=OracleMath())
 
 
+class _FailingForward:
+    """A forward whose kernels gave up on one rank."""
+
+    def __init__(self, fails):
+        self.fails = fails
+
+    def __call__(self, batch):
+        return _forward(batch)
+
+    def check_status(self):
+        if self.fails:
+            raise ArithmeticError("a wait ran out")
+
+
+def _failing_worker(rank, world, port, q):
+    os.environ["MASTER_ADDR"] = "127.0.0.1"
+    os.environ["MASTER_PORT"] = str(port)
+    dist.init_process_group("gloo", rank=rank, world_size=world)
+    samples = _make_samples(4)
+    try:
+        ShardedCalibrator(_FailingForward(rank == 1), math=OracleMath(), dist=dist).run([samples[2 * rank:2 * rank + 2]], samples_per_rank=2)
+        q.put((rank, None))
+    except Exception as e:
+        q.put((rank, type(e).__name__))
+    dist.barrier()
+    dist.destroy_process_group()
+
+
+def test_a_forward_that_failed_is_reported_on_every_rank():
+    cal = ShardedCalibrator(_FailingForward(True), math=OracleMath(), dist=None)
+    with pytest.raises(ArithmeticError):
+        cal.run([_make_samples(3)], samples_per_rank=3)
+    with socket.socket() as s:
+        s.bind(("127.0.0.1", 0))
+        port = s.getsockname()[1]
+    ctx = mp.get_context("spawn")
+    q = ctx.Queue()
+    procs = [ctx.Process(target=_failing_worker, args=(r, 2, port, q)) for r in range(2)]
+    for p in procs:
+        p.start()
+    got = dict(q.get(timeout=120) for _ in procs)
+    for p in procs:
+        p.join(timeout=60)
+        assert p.exitcode == 0
+    assert got == {0: "RuntimeError", 1: "ArithmeticError"}
+
+
 def test_single_process_path():
     samples = _make_samples(6)
     cal = ShardedCalibrator(_forward, math=OracleMath(), dist=None)

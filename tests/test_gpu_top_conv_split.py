@@ -213,3 +213,50 @@ def test_capture_and_two_streams():
                 outs[i].append(conv(x if i == 0 else x2))
     torch.cuda.synchronize()
     assert all(torch.equal(o, want) for o in outs[0]) and all(torch.equal(o, want2) for o in outs[1])
+
+
+@pytest.mark.parametrize("case", [CASES[i] for i in (0, 4, 6, 9)])       # 64 wide, strided, split, pair
+def test_a_wait_that_runs_out_is_reported(case):
+    """Failure detection without a fault: every stage's barrier is told to expect 16 bytes more than the loads deliver, so a bounded
+    wait runs out after 1 ms.  With a split and a ReLU the lost sums end as zeros: only the status tells."""
+    n, ic, ih, iw, oc, kh, kw, stride, pads, dil = case
+    x, w, b = draw(1, n, ic, ih, iw, oc, kh, kw)
+    conv = Conv(w, b, ih, iw, stride, pads, dil, True)
+    want, lib = conv(x), L.lib()
+    assert lib.b200q_top_conv2d_dev_status(conv.h, None) == L.OK
+    lib.b200q_debug_set_wait_fault(16, 1_000_000)
+    try:
+        conv(x)
+        rc = lib.b200q_top_conv2d_dev_status(conv.h, None)
+    finally:
+        lib.b200q_debug_set_wait_fault(0, 0)
+    assert rc == L.ERR_TIMEOUT
+    assert torch.equal(conv(x), want) and lib.b200q_top_conv2d_dev_status(conv.h, None) == L.OK
+
+
+def test_executor_and_calibration_report_it():
+    from tpu_mlir_b200.module import module
+    from tpu_mlir_b200.run_calibration import run_calibration
+    rng = np.random.default_rng(0)
+    shape = dict(shape=[2, 32, 12, 12], dtype="f32")
+    conv = dict(kernel_shape=[3, 3], pads=[1, 1, 1, 1], do_relu=True)
+    graph = dict(inputs=["x"], outputs=["c2"], tensors=dict(x=shape, c1=shape, c2=shape), state="TOP_F32",
+                 ops=[dict(type="top.Conv", name="c1", inputs=["x"], attrs=conv), dict(type="top.Conv", name="c2", inputs=["c1"], attrs=conv)])
+    weights = {f"{c}_{k}": rng.standard_normal(s).astype(np.float32) for c in ("c1", "c2") for k, s in (("filter", (32, 32, 3, 3)), ("bias", (32,)))}
+    samples = rng.standard_normal((4, 32, 12, 12)).astype(np.float32)
+    m, lib = module(), L.lib()
+    m.load(graph, weights)
+    m.set_tensor("x", samples[:2])
+    lib.b200q_debug_set_wait_fault(16, 1_000_000)
+    try:
+        m.invoke()
+        with pytest.raises(L.B200QError) as e:
+            m.check_status()
+        assert e.value.code == L.ERR_TIMEOUT
+        with pytest.raises(L.B200QError):
+            run_calibration(graph, weights, samples)
+    finally:
+        lib.b200q_debug_set_wait_fault(0, 0)
+    m.invoke()
+    m.check_status()
+    assert len(run_calibration(graph, weights, samples)) == 3

@@ -148,6 +148,8 @@ SIGNATURES = {
     "b200q_top_conv2d_dev_create": (C.c_int, [C.POINTER(TopConvDesc), C.c_void_p, C.c_void_p, _VPP]),
     "b200q_top_conv2d_dev_run": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
     "b200q_top_conv2d_dev_output_shape": (None, [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
+    "b200q_top_conv2d_dev_status": (C.c_int, [C.c_void_p, C.c_void_p]),
+    "b200q_top_conv2d_dev_set_status": (C.c_int, [C.c_void_p, C.c_void_p]),
     "b200q_top_conv2d_dev_destroy": (None, [_VPP]),
     "b200q_top_matmul_f32_dev": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64,
                                            C.c_int32, C.c_float, C.c_void_p]),

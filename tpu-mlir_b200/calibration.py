@@ -265,7 +265,8 @@ class ShardedCalibrator:
     """Statistics + KLD thresholds for the activations of a forward function, samples sharded across ranks.
 
     ``forward(batch) -> dict name -> device float32 tensor [B, ...]`` produces every activation of interest for a
-    batch of samples; ``shard`` is the local contiguous range of the global sample order.  ``math`` defaults to
+    batch of samples; if it has a ``check_status``, that is called once after the last batch and raises if a kernel gave up
+    (min / max and the histogram pass over NaN, so a lost activation would end as a plausible threshold); ``shard`` is the local contiguous range of the global sample order.  ``math`` defaults to
     the GPU implementation; ``dist`` is a torch.distributed-like module (None = single process).
     """
 
@@ -275,6 +276,22 @@ class ShardedCalibrator:
         self.dist = dist if (dist is not None and dist.is_initialized() and dist.get_world_size() > 1) else None
         self.bin_num = bin_num
         self.dst_bins = dst_bins
+
+    def _check_forward(self, device):
+        """Raises on every rank if the forward of one reports that its activations are not valid."""
+        import torch
+        failed = None
+        try:
+            getattr(self.forward, "check_status", lambda: None)()
+        except Exception as e:      # the ranks learn of it from each other before the next collective
+            failed = e
+        if self.dist:
+            count = torch.tensor([int(failed is not None)], dtype=torch.int32, device=device)
+            self.dist.all_reduce(count)
+            if failed is None and int(count.item()):
+                raise RuntimeError(f"the forward of {int(count.item())} other rank(s) failed")
+        if failed is not None:
+            raise failed
 
     def _world(self):
         return (self.dist.get_rank(), self.dist.get_world_size()) if self.dist else (0, 1)
@@ -426,6 +443,7 @@ class ShardedCalibrator:
             done += next(iter(acts.values())).shape[0]
             del acts
         store = None
+        self._check_forward(mm_local.device)
         t0 = lap("pass2_histograms", t0)
         # this rank's own contribution, kept for save_shard (the all-reduce below overwrites `flat` with the sum)
         self._shard = dict(names=list(names), minmax=mm_local.cpu().numpy(), hist=flat.cpu().numpy().copy(), sizes=np.asarray(sizes, np.int64),
@@ -513,6 +531,7 @@ class ShardedCalibrator:
             done += B
             del acts, xs
         assert done == samples, "batches do not cover samples_per_rank samples"
+        self._check_forward(m.device)
         t0 = lap("pass_forward_statistics", t0)
         st = sched.state
         views = {n: own.get(t, rows[t])[:max(int(st["bins"][t]), 1)] for t, n in enumerate(names)}

@@ -71,6 +71,8 @@ struct TopConvHandle {
   PoolRef scratch;
   DevBuf wt, ktab, bias, w_stage, x, y, ws;
   DevBuf planes;                   // the weight as three bf16 planes, where the tensor-core form applies
+  DevBuf status;                   // its wait site, unless the caller named a word
+  int* d_status = nullptr;
   bool with_bias = false;
   const float* d_bias = nullptr;   // device face: the caller's
 };
@@ -119,7 +121,12 @@ int b200q_top_conv2d_dev_create(const b200q_top_conv_desc* desc, const float* fi
   if (rc == B200Q_OK && top_conv_umma_takes(p) && cudaGetDevice(&h->scratch.dev) == cudaSuccess) {
     if (h->planes.ensure(top_conv_umma_weight_bytes(p)) == B200Q_OK) h->scratch.pool = pool_acquire(h->scratch.dev);
     else cudaGetLastError();       // no room for the planes: the CUDA-core kernel serves this layer
-    if (h->scratch.pool) rc = top_conv_umma_prepare(p, filter_oihw, h->planes.p, 0);
+    if (h->scratch.pool) {
+      rc = top_conv_umma_prepare(p, filter_oihw, h->planes.p, 0);
+      if (rc == B200Q_OK) rc = h->status.ensure(4);
+      if (rc == B200Q_OK && cudaMemsetAsync(h->status.p, 0, 4, 0) != cudaSuccess) rc = cuda_error(cudaGetLastError(), "memset", __FILE__, __LINE__);
+      h->d_status = h->status.as<int>();
+    }
   }
   if (rc == B200Q_OK && cudaStreamSynchronize(0) != cudaSuccess) rc = cuda_error(cudaGetLastError(), "sync", __FILE__, __LINE__);
   if (rc != B200Q_OK) {
@@ -142,7 +149,7 @@ int b200q_top_conv2d_dev_run(void* handle, const float* x, float* y, int64_t bat
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     void* scratch = nullptr;
     if (cudaMallocFromPoolAsync(&scratch, top_conv_umma_scratch(p, sms), h->scratch.pool, s) == cudaSuccess) {
-      const int rc = top_conv_umma_launch(p, x, h->wt.as<float>(), h->planes.p, h->d_bias, y, scratch, sms, s);
+      const int rc = top_conv_umma_launch(p, x, h->wt.as<float>(), h->planes.p, h->d_bias, y, scratch, h->d_status, sms, s);
       const cudaError_t e = cudaFreeAsync(scratch, s);
       if (rc == B200Q_OK && e != cudaSuccess) return cuda_error(e, "cudaFreeAsync", __FILE__, __LINE__);
       return rc;
@@ -152,6 +159,25 @@ int b200q_top_conv2d_dev_run(void* handle, const float* x, float* y, int64_t bat
   p.splits = top_conv_splits(p, sms);
   if (p.splits > 1) B200Q_TRY(h->ws.ensure((size_t)p.splits * p.n * p.oc * p.oh * p.ow * 4));   // grows on the first call of a batch size
   return top_conv_launch(p, x, h->wt.as<float>(), h->ktab.as<int2>(), h->d_bias, y, h->ws.as<float>(), static_cast<cudaStream_t>(stream));
+}
+
+int b200q_top_conv2d_dev_set_status(void* handle, int32_t* status) {
+  if (!handle) return set_error(B200Q_ERR_INVALID, "top_conv2d_dev_set_status: null handle");
+  TopConvHandle* h = static_cast<TopConvHandle*>(handle);
+  if (h->scratch.pool) h->d_status = status ? status : h->status.as<int>();
+  return B200Q_OK;
+}
+
+int b200q_top_conv2d_dev_status(void* handle, void* stream) {
+  if (!handle) return set_error(B200Q_ERR_INVALID, "top_conv2d_dev_status: null handle");
+  TopConvHandle* h = static_cast<TopConvHandle*>(handle);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  int code = 0;
+  if (h->d_status) CUDA_TRY(cudaMemcpyAsync(&code, h->d_status, 4, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaStreamSynchronize(s));
+  if (code == 0) return B200Q_OK;
+  CUDA_TRY(cudaMemsetAsync(h->d_status, 0, 4, s));
+  return set_error(B200Q_ERR_TIMEOUT, "top conv: a bounded wait inside the kernel ran out (wait site %d)", code);
 }
 
 void b200q_top_conv2d_dev_output_shape(void* handle, int64_t* oh, int64_t* ow) {

@@ -72,6 +72,7 @@ int make_tmap_u8(CUtensorMap* map, const void* base, int rank, const uint64_t* d
 int igemm_i8_tcgen05_supported(const IGemmProblem& p, const char** why);
 int igemm_i8_tcgen05_launch(const IGemmProblem& p, const Epilogue& epi, int* status, cudaStream_t stream);
 void igemm_set_wait_test(int extra_tx_bytes, long long budget_ns);
+void igemm_wait_test(int* extra_tx_bytes, unsigned long long* budget_ns);   // what the tensor-core launches use
 // Plain CUDA-core kernel for shapes the tensor-core path does not take (odd K, strides, groups, dilation).
 struct ConvGeometry {
   int n, ic, ih, iw, oc, oh, ow, kh, kw, sh, sw, dh, dw, pht, pwl, groups, pad_value;

@@ -957,6 +957,11 @@ void igemm_set_wait_test(int extra_tx_bytes, long long budget_ns) {
   g_wait_budget_ns.store(budget_ns > 0 ? (unsigned long long)budget_ns : DEFAULT_WAIT_BUDGET_NS, std::memory_order_relaxed);
 }
 
+void igemm_wait_test(int* extra_tx_bytes, unsigned long long* budget_ns) {
+  *extra_tx_bytes = g_expect_extra.load(std::memory_order_relaxed);
+  *budget_ns = g_wait_budget_ns.load(std::memory_order_relaxed);
+}
+
 static bool tapfuse_allowed() {
   static const bool on = [] {
     const char* v = getenv("B200Q_IGEMM_TAPFUSE");
@@ -1037,8 +1042,7 @@ int igemm_i8_tcgen05_launch(const IGemmProblem& p, const Epilogue& epi, int* sta
     a.add_lo = p.add_lo;
     a.add_hi = p.add_hi;
   }
-  a.wait_budget_ns = g_wait_budget_ns.load(std::memory_order_relaxed);
-  a.expect_extra = g_expect_extra.load(std::memory_order_relaxed);
+  igemm_wait_test(&a.expect_extra, &a.wait_budget_ns);
   a.bf16 = p.kind == IGEMM_KIND_BF16 || p.kind == IGEMM_KIND_F16;
   a.f16 = p.kind == IGEMM_KIND_F16;
   // |accumulator| < 2^29 for every 8-bit operand pair: lets the epilogue fold the bias into one 64-bit constant

@@ -28,13 +28,13 @@ int top_conv_reduce_launch(const float* planes, const float* bias, float* y, lon
                            float relu_limit, cudaStream_t s);
 // The same convolution on the tensor cores (top_f32_umma.cu).  takes: whether a plan of one image or more qualifies; prepare:
 // once per handle, the weight's bf16 planes (weight_bytes of them); launch: `scratch` holds top_conv_umma_scratch bytes and is
-// free again when the stream has passed the call.
+// free again when the stream has passed the call; *status (device) gets the wait site if a bounded wait runs out.
 bool top_conv_umma_takes(const TopConvPlan& p);
 size_t top_conv_umma_weight_bytes(const TopConvPlan& p);
 int top_conv_umma_prepare(const TopConvPlan& p, const float* w_oihw, void* planes, cudaStream_t s);
 size_t top_conv_umma_scratch(const TopConvPlan& p, int sms);
 int top_conv_umma_launch(const TopConvPlan& p, const float* x, const float* wt, const void* w_planes, const float* bias, float* y,
-                         void* scratch, int sms, cudaStream_t s);
+                         void* scratch, int* status, int sms, cudaStream_t s);
 // y[M][N] = relu(x[M][K] * w[K][N] + bias)
 int top_matmul_launch(const float* x, const float* w_kn, const float* bias, float* y, int M, int K, int N, int do_relu, float relu_limit,
                       int sms, cudaStream_t s);

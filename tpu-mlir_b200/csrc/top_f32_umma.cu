@@ -45,7 +45,6 @@ constexpr int PARTS = 2;                       // accumulators of a chunk: the s
 constexpr int CHUNK_BYTES = CHUNK * 2;
 constexpr int A_STAGES = 2;
 constexpr int MAX_SHARE = 3;
-constexpr uint64_t WAIT_BUDGET_NS = 2000000000ull;
 
 // BN: channels of a tile.  PAIR: two CTAs of a cluster compute 256 rows x BN channels (tcgen05 cta_group::2); each loads its
 // own 128 rows of A and half of B.
@@ -61,7 +60,7 @@ struct UmmaLayout {
   static constexpr int B_BYTES = 3 * B_PLANE;
   static constexpr int B_OFFSET = A_STAGES * A_BYTES;
   static constexpr int BAR_OFFSET = B_OFFSET + B_STAGES * B_BYTES;
-  static constexpr int MISC_OFFSET = BAR_OFFSET + (2 * A_STAGES + 2 * B_STAGES + 2 * BUFS) * 8;
+  static constexpr int MISC_OFFSET = BAR_OFFSET + (2 * A_STAGES + 2 * B_STAGES + 2 * BUFS + 1) * 8;
   static constexpr int DYN_BYTES = MISC_OFFSET + 16 + 1024;      // slack for the manual 1024-byte alignment
   static constexpr int EPI_WARPS = BN == 64 ? 8 : 16;
   static constexpr int EPI_COLS = BN * 4 / EPI_WARPS;            // a warp: 32 rows x 32 channels (64 at BN = 256)
@@ -231,6 +230,9 @@ struct UmmaArgs {
   const uint32_t* w_range;   // [oc]
   float k_total;             // products of one output
   int x_blocks, x_groups, halo;   // halo: rows past a tile's last that its last row's taps reach
+  int* status;               // set to the wait site if a bounded wait ran out; the results are not valid then
+  unsigned long long wait_budget_ns;
+  int expect_extra;          // test aid: bytes a stage's barrier expects beyond what its loads deliver (0 in normal use)
 };
 
 // Units [u0, u1) of k as runs of channels of one tap: f(tap, first channel, end), until it returns false
@@ -299,6 +301,12 @@ __device__ __noinline__ void recompute(const UmmaArgs& a, int row, int co, int s
   }
 }
 
+// Waits until the phase is complete, but not for long: what is on its way here arrives within microseconds.
+__device__ __forceinline__ void drain(uint32_t bar, uint32_t parity) {
+  const uint64_t t0 = ptx::globaltimer_ns();
+  while (!ptx::mbar_try_wait_hint(bar, parity, 20000u) && ptx::globaltimer_ns() - t0 < 200000u) {}
+}
+
 template <int BN, bool PAIR>
 __global__ void __launch_bounds__(UmmaLayout<BN, PAIR>::THREADS, 1)
 conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ UmmaArgs args) {
@@ -313,6 +321,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   auto empty_b = [&](int s) { return bar_base + 8u * (2 * A_STAGES + L::B_STAGES + s); };
   auto tmem_full_bar = [&](int b) { return bar_base + 8u * (2 * A_STAGES + 2 * L::B_STAGES + b); };
   auto tmem_empty_bar = [&](int b) { return bar_base + 8u * (2 * A_STAGES + 2 * L::B_STAGES + L::BUFS + b); };
+  const uint32_t mma_done_bar = bar_base + 8u * (2 * A_STAGES + 2 * L::B_STAGES + 2 * L::BUFS);   // used after a wait ran out
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::MISC_OFFSET);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::MISC_OFFSET + 4);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -334,6 +343,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       ptx::mbar_init(tmem_full_bar(b), 1);
       ptx::mbar_init(tmem_empty_bar(b), CTAS * L::EPI_WARPS);
     }
+    ptx::mbar_init(mma_done_bar, 1);
     *abort_flag = 0;
     ptx::fence_barrier_init();
     ptx::fence_proxy_async_smem();
@@ -374,12 +384,12 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         int group = u0 / args.units_per_tap, kc = u0 - group * args.units_per_tap;
         for (int u = u0; u < u1 && ok; ++u) {
           if (warp == 0) {
-            ok = ptx::mbar_wait_bounded_fast<20>(empty_a(stage), phase ^ 1u, abort_flag, 1, WAIT_BUDGET_NS);
+            ok = ptx::mbar_wait_bounded_fast<20>(empty_a(stage), phase ^ 1u, abort_flag, 1, args.wait_budget_ns);
             if (!ok) break;
             const int fy = group / args.taps_w, fx = group - fy * args.taps_w;
             const int row = mt * (CTAS * TILE_M) + (int)rank * TILE_M + fy * args.tap_h + fx * args.tap_w;
             const uint32_t sa = smem_base + stage * L::A_BYTES;
-            if (rank == 0) ptx::mbar_arrive_expect_tx(full_a(stage), CTAS * 3 * (TILE_M + share - 1) * CHUNK_BYTES);
+            if (rank == 0) ptx::mbar_arrive_expect_tx(full_a(stage), CTAS * 3 * (TILE_M + share - 1) * CHUNK_BYTES + args.expect_extra);
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
               if (PAIR) ptx::tma_load_3d_pair(sa + q * L::A_PLANE, &tmap_a, ptx::map_to_cta(full_a(stage), 0), kc * CHUNK_BYTES, row, q);
@@ -391,7 +401,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             }
           } else {
             for (int t = 0; t < share; ++t) {
-              ok = ptx::mbar_wait_bounded_fast<20>(empty_b(stage), phase ^ 1u, abort_flag, 2, WAIT_BUDGET_NS);
+              ok = ptx::mbar_wait_bounded_fast<20>(empty_b(stage), phase ^ 1u, abort_flag, 2, args.wait_budget_ns);
               if (!ok) break;
               const int col = (group * share + t) * args.tap_k * 2 + kc * CHUNK_BYTES;
               const uint32_t sb = smem_base + L::B_OFFSET + stage * L::B_BYTES;
@@ -409,6 +419,12 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             ++group;
           }
         }
+      }
+      if (!ok && rank == 0) {
+        // a wait ran out: do not leave while copies of this pair may still be on their way (stages from `stage` on were last
+        // filled in the phase before)
+        const int stages = warp == 0 ? A_STAGES : L::B_STAGES;
+        for (int i = 0; i < stages; ++i) drain(warp == 0 ? full_a(i) : full_b(i), i < stage ? phase : phase ^ 1u);
       }
     }
   } else if (warp == 1) {
@@ -432,15 +448,15 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         const int split = tile / args.n_tiles / args.m_tiles;
         const int u0 = split * args.units_per_split, u1 = min(args.units, u0 + args.units_per_split);
         for (int u = u0; u < u1 && ok; ++u) {
-          ok = ptx::mbar_wait_bounded_fast<20>(full_a(sa), pa, abort_flag, 3, WAIT_BUDGET_NS);
+          ok = ptx::mbar_wait_bounded_fast<20>(full_a(sa), pa, abort_flag, 3, args.wait_budget_ns);
           for (int t = 0; t < share && ok; ++t) {
-            ok = ptx::mbar_wait_bounded_fast<20>(full_b(sb), pb, abort_flag, 5, WAIT_BUDGET_NS);
+            ok = ptx::mbar_wait_bounded_fast<20>(full_b(sb), pb, abort_flag, 5, args.wait_budget_ns);
             // tap t reads the block from row t on: the swizzle follows the address bits, only the start moves
             const uint32_t al = a_lo0 + (uint32_t)(sa * (L::A_BYTES >> 4) + t * (CHUNK_BYTES >> 4));
             const uint32_t bl = b_lo0 + (uint32_t)(sb * (L::B_BYTES >> 4));
 #pragma unroll
             for (int part = 0; part < PARTS && ok; ++part) {
-              ok = ptx::mbar_wait_bounded_fast<20>(tmem_empty_bar(buf), buf_phase ^ 1u, abort_flag, 4, WAIT_BUDGET_NS);
+              ok = ptx::mbar_wait_bounded_fast<20>(tmem_empty_bar(buf), buf_phase ^ 1u, abort_flag, 4, args.wait_budget_ns);
               if (!ok) break;
               ptx::tc_fence_after_sync();
               const uint32_t d = tmem_base + (uint32_t)(buf * BN);
@@ -473,6 +489,11 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             pa ^= 1u;
           }
         }
+      }
+      if (!ok) {   // nor while products are being written to the tensor memory that is freed below
+        if (PAIR) ptx::umma_commit_pair(mma_done_bar, 1);
+        else ptx::umma_commit(mma_done_bar);
+        drain(mma_done_bar, 0u);
       }
     }
   } else {
@@ -518,7 +539,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       for (int j = 0; j < L::EPI_COLS; ++j) acc[j] = 0.f;
       const int sums = (u1 - u0) * share * PARTS;
       for (int q = 0; q < sums && ok; ++q) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded_fast<20>(tmem_full_bar(buf), buf_phase, abort_flag, 6, WAIT_BUDGET_NS));
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait_bounded_fast<20>(tmem_full_bar(buf), buf_phase, abort_flag, 6, args.wait_budget_ns));
         if (!ok) break;
         ptx::tc_fence_after_sync();
 #pragma unroll
@@ -573,7 +594,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           asm volatile("" : "+l"(o));   // one running address: 64 of them kept ahead spilled the sums
         }
       }
-      // the rare ones, and everything if a wait ran out (the sums are lost, and say so)
+      // the rare ones, and everything if a wait ran out (the sums are lost: NaN, and the status word)
 #pragma unroll
       for (int i = 0; i < L::EPI_COLS / 32; ++i) {
         if (!ok) {
@@ -587,6 +608,7 @@ conv_f32_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   if (PAIR && *abort_flag != 0) ptx::st_shared_cluster_u32(ptx::map_to_cta(ptx::smem_u32((const void*)abort_flag), rank ^ 1u), (uint32_t)*abort_flag);
   ptx::tc_fence_before_sync();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0 && args.status != nullptr) atomicCAS(args.status, 0, *abort_flag);
   if (PAIR) ptx::cluster_sync_all();   // neither CTA frees tensor memory or exits while the other can still signal or read it
   if (warp == 1) {
     ptx::tc_fence_after_sync();
@@ -737,7 +759,7 @@ size_t top_conv_umma_scratch(const TopConvPlan& p, int sms) {
 }
 
 int top_conv_umma_launch(const TopConvPlan& plan, const float* x, const float* wt, const void* w_planes, const float* bias, float* y,
-                         void* scratch, int sms, cudaStream_t s) {
+                         void* scratch, int* status, int sms, cudaStream_t s) {
   const int g = group_images(plan), cp = cp_of(plan), taps = plan.kh * plan.kw;
   const bool shifted = shifted_rows(plan);
   const UmmaChoice c = choose(plan, g, sms);
@@ -789,6 +811,8 @@ int top_conv_umma_launch(const TopConvPlan& plan, const float* x, const float* w
     a.x_groups = (int)(grid.y * grid.z);
     a.halo = shifted ? (p.kh - 1) * a.tap_h + (p.kw - 1) * a.tap_w : 0;
     a.k_total = (float)taps * (float)p.ic;
+    a.status = status;
+    igemm_wait_test(&a.expect_extra, &a.wait_budget_ns);
 
     CUtensorMap ta, tb;
     {

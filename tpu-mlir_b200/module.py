@@ -114,6 +114,9 @@ class module:  # noqa: N801  (name of the reference class)
     def _build_plans(self):
         self._release_handles()
         self._plans, self._keep, self._status, self._graph = [], [], [], None
+        # status words of the fp32 convolutions, read together: one per op of the graph
+        self._top_status = self.torch.zeros(len(self.graph["ops"]), dtype=self.torch.int32, device=self.device)
+        self._top_names: List[str] = []
         self._fuse_into, self._fused_adds = self._find_residual_adds() if self.fuse_residual_add else ({}, {})
         for op in self.graph["ops"]:
             self._plans.append(self._plan(op))
@@ -904,6 +907,8 @@ class module:  # noqa: N801  (name of the reference class)
             h = C.c_void_p()
             L.check(lib.b200q_top_conv2d_dev_create(C.byref(d), _P(w), _P(b), C.byref(h)))
             self._top_handles.append(h)
+            L.check(lib.b200q_top_conv2d_dev_set_status(h, _P(self._top_status[len(self._top_names):])))
+            self._top_names.append(op["name"])
             self._keep.append((w, b))
             return lambda: L.check(lib.b200q_top_conv2d_dev_run(h, _P(ins[0]), _P(out), n, stream()))
         if t == "top.MatMul":
@@ -1145,6 +1150,12 @@ class module:  # noqa: N801  (name of the reference class)
         """Raises B200QError(ERR_TIMEOUT) if a bounded wait inside one of the graph's tensor-core kernels ran out
         during an earlier invoke (the kernel returns early then and its output is not valid)."""
         self.torch.cuda.synchronize(self.device)
+        if self._top_names:
+            codes = self._top_status.tolist()
+            if any(codes):
+                self._top_status.zero_()
+                bad = [i for i, c in enumerate(codes) if c]
+                raise L.B200QError(L.ERR_TIMEOUT, f"{self._top_names[bad[0]]}: a bounded wait inside the kernel ran out (wait site {codes[bad[0]]})")
         for name, st in self._status:
             if isinstance(st, C.c_void_p):
                 rc = self.lib.b200q_conv2d_dev_status(st, None)

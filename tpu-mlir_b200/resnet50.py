@@ -71,6 +71,7 @@ class Fp32Forward:
         self.shape = {}
         with torch.cuda.device(self.device):
             shapes = {"input": (3, 224, 224)}
+            self._status = torch.zeros(len(ops), dtype=torch.int32, device=self.device)     # one word per convolution
             for op in ops:
                 cin = shapes[op["inputs"][0]]
                 if op["type"] == "conv":
@@ -85,6 +86,7 @@ class Fp32Forward:
                                                                 C.byref(h)))
                     oh, ow = C.c_int64(), C.c_int64()
                     L.lib().b200q_top_conv2d_dev_output_shape(h, C.byref(oh), C.byref(ow))
+                    L.check(L.lib().b200q_top_conv2d_dev_set_status(h, C.c_void_p(self._status[len(self.handles):].data_ptr())))
                     self.handles[op["name"]] = h
                     self.par[op["name"]] = (w, b)          # the handle reads the bias in place: keep it alive
                     shapes[op["name"]] = (oc, oh.value, ow.value)
@@ -110,6 +112,15 @@ class Fp32Forward:
                 self.L.lib().b200q_top_conv2d_dev_destroy(self.C.byref(h))
         except Exception:
             pass
+
+    def check_status(self):
+        """Raises B200QError(ERR_TIMEOUT) if a bounded wait inside a convolution ran out (its activations are not valid)."""
+        self.torch.cuda.synchronize(self.device)
+        codes = self._status.tolist()
+        if any(codes):
+            self._status.zero_()
+            i = next(i for i, c in enumerate(codes) if c)
+            raise self.L.B200QError(self.L.ERR_TIMEOUT, f"{list(self.handles)[i]}: a bounded wait inside the kernel ran out (wait site {codes[i]})")
 
     def __call__(self, x) -> Dict[str, "object"]:
         torch, C, L = self.torch, self.C, self.L

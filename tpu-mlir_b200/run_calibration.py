@@ -49,6 +49,8 @@ def run_calibration(graph, weights, samples, *, tune_num: int = 0, out_table: Op
         m.invoke()
         return {n: m._nchw(n) if n in m._nhwc else m.tensors[n] for n in names}
 
+    forward.check_status = m.check_status
+
     class Batches:      # re-iterable: the calibrator walks the samples twice
         def __iter__(self):
             return (local[i:i + batch] for i in range(0, per_rank, batch))

@@ -138,4 +138,6 @@ class SimpleTuner:
                 if tuned_op not in self.tuned_op_list:
                     self.find_better_threshold(evaled_op, tuned_op)
                     self.tuned_op_list.append(tuned_op)
+        self.module.check_status()
+        self.module_dq.check_status()
         return dict(self.thresholds)
