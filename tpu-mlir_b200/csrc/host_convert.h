@@ -1,0 +1,15 @@
+// The interpreter keeps every tensor as float: its integers in float buffers <-> their storage types, on host memory.
+#pragma once
+#include <stddef.h>
+#include <stdint.h>
+
+namespace b200q {
+
+// y[i] = (uint8_t)(int)x[i]: integral by contract, so the low byte is the int8 or uint8 value
+void host_f32_to_bytes(const float* x, uint8_t* y, size_t n);
+// y[i] = (float)x[i] for the storage type `dt` (b200q_dtype)
+void host_q_to_f32(const void* x, int dt, float* y, size_t n);
+// a short rest in a polling loop
+void host_pause();
+
+}  // namespace b200q

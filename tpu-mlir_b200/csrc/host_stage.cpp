@@ -9,7 +9,6 @@
 // copied, 0.47 ms this way.
 #include "host_stage.h"
 
-#include <immintrin.h>
 #include <sched.h>
 #include <string.h>
 
@@ -22,77 +21,7 @@ constexpr int MAX_SLOTS = 4;                     // pieces in flight: bounds the
 constexpr size_t INLINE_VALUES = 96 * 1024;      // up to here the calling thread converts alone: a wake-up costs as much
 constexpr size_t STREAM_STORE_VALUES = 512 * 1024;
 
-void f32_to_bytes_scalar(const float* x, uint8_t* y, size_t n) {
-  for (size_t i = 0; i < n; ++i) y[i] = (uint8_t)(int)x[i];
-}
-
-__attribute__((target("avx2"))) void f32_to_bytes_avx2(const float* x, uint8_t* y, size_t n) {
-  const __m256i low = _mm256_set1_epi32(0xff);
-  const __m256i order = _mm256_setr_epi32(0, 4, 1, 5, 2, 6, 3, 7);   // undo the per-128-bit-lane packing
-  size_t i = 0;
-  for (; i + 32 <= n; i += 32) {
-    const __m256i a = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i)), low);
-    const __m256i b = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i + 8)), low);
-    const __m256i c = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i + 16)), low);
-    const __m256i d = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i + 24)), low);
-    const __m256i p = _mm256_packus_epi16(_mm256_packus_epi32(a, b), _mm256_packus_epi32(c, d));
-    _mm256_storeu_si256(reinterpret_cast<__m256i*>(y + i), _mm256_permutevar8x32_epi32(p, order));
-  }
-  f32_to_bytes_scalar(x + i, y + i, n - i);
-}
-
-template <typename T>
-void q_to_f32_scalar(const T* x, float* y, size_t n) {
-  for (size_t i = 0; i < n; ++i) y[i] = (float)x[i];
-}
-
-// 8-bit to float, 32 values per step; the output is written past the caches (it is four times the input and read by
-// nobody in this call)
-template <bool SIGNED>
-__attribute__((target("avx2"))) void bytes_to_f32_avx2(const uint8_t* x, float* y, size_t n) {
-  size_t i = 0;
-  while (i < n && (reinterpret_cast<uintptr_t>(y + i) & 31) != 0) {
-    y[i] = SIGNED ? (float)(int8_t)x[i] : (float)x[i];
-    ++i;
-  }
-  for (; i + 32 <= n; i += 32) {
-    for (int k = 0; k < 4; ++k) {
-      const __m128i b = _mm_loadl_epi64(reinterpret_cast<const __m128i*>(x + i + 8 * k));
-      const __m256i w = SIGNED ? _mm256_cvtepi8_epi32(b) : _mm256_cvtepu8_epi32(b);
-      _mm256_stream_ps(y + i + 8 * k, _mm256_cvtepi32_ps(w));
-    }
-  }
-  for (; i < n; ++i) y[i] = SIGNED ? (float)(int8_t)x[i] : (float)x[i];
-  _mm_sfence();
-}
-
-bool have_avx2() {
-  static const bool yes = __builtin_cpu_supports("avx2");
-  return yes;
-}
-
 }  // namespace
-
-void host_f32_to_bytes(const float* x, uint8_t* y, size_t n) {
-  if (have_avx2()) f32_to_bytes_avx2(x, y, n);
-  else f32_to_bytes_scalar(x, y, n);
-}
-
-void host_q_to_f32(const void* x, int dt, float* y, size_t n) {
-  switch (dt) {
-    case B200Q_DT_I8:
-      if (have_avx2()) bytes_to_f32_avx2<true>(static_cast<const uint8_t*>(x), y, n);
-      else q_to_f32_scalar(static_cast<const int8_t*>(x), y, n);
-      break;
-    case B200Q_DT_U8:
-      if (have_avx2()) bytes_to_f32_avx2<false>(static_cast<const uint8_t*>(x), y, n);
-      else q_to_f32_scalar(static_cast<const uint8_t*>(x), y, n);
-      break;
-    case B200Q_DT_I16: q_to_f32_scalar(static_cast<const int16_t*>(x), y, n); break;
-    case B200Q_DT_U16: q_to_f32_scalar(static_cast<const uint16_t*>(x), y, n); break;
-    default: q_to_f32_scalar(static_cast<const int32_t*>(x), y, n); break;
-  }
-}
 
 // ---------------------------------------------------------------------------------------------- HostPool
 std::shared_ptr<HostPool> HostPool::get() {
@@ -163,7 +92,7 @@ void HostPool::loop() {
     bool ran = false;
     for (int spin = 0; spin < 2000 && !ran; ++spin) {
       ran = help();
-      if (!ran) _mm_pause();
+      if (!ran) host_pause();
     }
     if (ran) continue;
     std::unique_lock<std::mutex> lock(m_);
@@ -266,7 +195,7 @@ void HostStage::convert(const void* src, void* dst, size_t n, int dt, size_t out
     tasks.push_back(HostTask{static_cast<const uint8_t*>(src) + o * ss, static_cast<uint8_t*>(dst) + o * ds, n - o < step ? n - o : step, dt, &left});
   pool_->submit(tasks.data(), tasks.size());
   while (left.load(std::memory_order_acquire) > 0)
-    if (!pool_->help()) _mm_pause();
+    if (!pool_->help()) host_pause();
 }
 
 int HostStage::run(const float* x, float* y, int64_t units, size_t x_per, size_t y_per, int out_dt, size_t out_size, int* status,
@@ -396,16 +325,16 @@ int HostStage::run_pieces(const float* x, float* y, int64_t units, int64_t per, 
       ++finished;
       moved = true;
     }
-    if (!moved && !pool_->help()) _mm_pause();
+    if (!moved && !pool_->help()) host_pause();
   }
   if (rc != B200Q_OK) {   // nothing of this call may still touch its buffers when it returns
     for (auto& st : streams_.s) cudaStreamSynchronize(st);
     for (int c = 0; c < submitted; ++c)
       while (in_left[(size_t)c].load(std::memory_order_acquire) > 0)
-        if (!pool_->help()) _mm_pause();
+        if (!pool_->help()) host_pause();
     for (int c = 0; c < drained; ++c)
       while (out_left[(size_t)c].load(std::memory_order_acquire) > 0)
-        if (!pool_->help()) _mm_pause();
+        if (!pool_->help()) host_pause();
     return rc;
   }
   memcpy(status, out_.p + ys * (size_t)slots, 4);

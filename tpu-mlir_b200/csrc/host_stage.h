@@ -15,14 +15,10 @@
 #include <vector>
 
 #include "devbuf.h"
+#include "host_convert.h"
 #include "internal.h"
 
 namespace b200q {
-
-// y[i] = (uint8_t)(int)x[i]: integral by contract, so the low byte is the int8 or uint8 value
-void host_f32_to_bytes(const float* x, uint8_t* y, size_t n);
-// y[i] = (float)x[i] for the storage type `dt` (b200q_dtype)
-void host_q_to_f32(const void* x, int dt, float* y, size_t n);
 
 // One conversion of at most a few hundred KB; `left` counts the unfinished tasks of its piece.
 struct HostTask {
