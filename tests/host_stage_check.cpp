@@ -38,7 +38,7 @@ static int checks_conversions() {
       for (size_t i = 0; i < raw.size(); ++i) raw[i] = (int32_t)(i * 2654435761u);
       for (size_t o : {0, 1, 5}) {
         std::vector<float> y(n + 8, -7.5f);
-        host_q_to_f32(raw.data(), dt, y.data() + o, n);
+        host_q_to_f32(raw.data(), dt, y.data() + o, n, (n & 1) != 0 && o != 1);
         for (size_t i = 0; i < n; ++i) {
           const float want = dt == B200Q_DT_I8    ? (float)reinterpret_cast<int8_t*>(raw.data())[i]
                              : dt == B200Q_DT_U8  ? (float)reinterpret_cast<uint8_t*>(raw.data())[i]

@@ -37,9 +37,8 @@ __attribute__((target("avx2"))) void f32_to_bytes_avx2(const float* x, uint8_t* 
   f32_to_bytes_scalar(x + i, y + i, n - i);
 }
 
-// 8-bit to float, 32 values per step; the output is written past the caches (it is four times the input and read by
-// nobody in this call)
-template <bool SIGNED>
+// 8-bit to float, 32 values per step
+template <bool SIGNED, bool PAST_CACHE>
 __attribute__((target("avx2"))) void bytes_to_f32_avx2(const uint8_t* x, float* y, size_t n) {
   size_t i = 0;
   while (i < n && (reinterpret_cast<uintptr_t>(y + i) & 31) != 0) {
@@ -50,11 +49,12 @@ __attribute__((target("avx2"))) void bytes_to_f32_avx2(const uint8_t* x, float* 
     for (int k = 0; k < 4; ++k) {
       const __m128i b = _mm_loadl_epi64(reinterpret_cast<const __m128i*>(x + i + 8 * k));
       const __m256i w = SIGNED ? _mm256_cvtepi8_epi32(b) : _mm256_cvtepu8_epi32(b);
-      _mm256_stream_ps(y + i + 8 * k, _mm256_cvtepi32_ps(w));
+      if (PAST_CACHE) _mm256_stream_ps(y + i + 8 * k, _mm256_cvtepi32_ps(w));
+      else _mm256_store_ps(y + i + 8 * k, _mm256_cvtepi32_ps(w));
     }
   }
   for (; i < n; ++i) y[i] = SIGNED ? (float)(int8_t)x[i] : (float)x[i];
-  _mm_sfence();
+  if (PAST_CACHE) _mm_sfence();
 }
 
 bool have_avx2() {
@@ -82,10 +82,15 @@ void host_f32_to_bytes(const float* x, uint8_t* y, size_t n) {
   f32_to_bytes_scalar(x, y, n);
 }
 
-void host_q_to_f32(const void* x, int dt, float* y, size_t n) {
+void host_q_to_f32(const void* x, int dt, float* y, size_t n, bool past_cache) {
 #ifdef B200Q_HOST_AVX2
-  if (dt == B200Q_DT_I8 && have_avx2()) return bytes_to_f32_avx2<true>(static_cast<const uint8_t*>(x), y, n);
-  if (dt == B200Q_DT_U8 && have_avx2()) return bytes_to_f32_avx2<false>(static_cast<const uint8_t*>(x), y, n);
+  if ((dt == B200Q_DT_I8 || dt == B200Q_DT_U8) && have_avx2()) {
+    auto* f = dt == B200Q_DT_I8 ? (past_cache ? bytes_to_f32_avx2<true, true> : bytes_to_f32_avx2<true, false>)
+                                : (past_cache ? bytes_to_f32_avx2<false, true> : bytes_to_f32_avx2<false, false>);
+    return f(static_cast<const uint8_t*>(x), y, n);
+  }
+#else
+  (void)past_cache;
 #endif
   switch (dt) {
     case B200Q_DT_I8: q_to_f32_scalar(static_cast<const int8_t*>(x), y, n); break;

@@ -27,9 +27,10 @@ struct HostTask {
   size_t n;
   int dt;       // < 0: float -> bytes, else q -> float of this storage type
   std::atomic<int>* left;
+  bool past_cache;
   void run() const {
     if (dt < 0) host_f32_to_bytes(static_cast<const float*>(src), static_cast<uint8_t*>(dst), n);
-    else host_q_to_f32(src, dt, static_cast<float*>(dst), n);
+    else host_q_to_f32(src, dt, static_cast<float*>(dst), n, past_cache);
     left->fetch_sub(1, std::memory_order_release);
   }
 };
@@ -91,7 +92,7 @@ class HostStage {
   int grow(HostPool::Pinned* b, size_t bytes);
   int run_pieces(const float* x, float* y, int64_t units, int64_t per, size_t x_per, size_t y_per, int out_dt, size_t out_size, int* status,
                  const Launch& launch);
-  void convert(const void* src, void* dst, size_t n, int dt, size_t out_size, bool alone);
+  void convert(const void* src, void* dst, size_t n, int dt, size_t out_size, bool alone);   // of a call of one piece
   std::shared_ptr<HostPool> pool_;
   HostPool::Pinned in_, out_;
   HostPool::Streams streams_;
