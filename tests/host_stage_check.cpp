@@ -7,6 +7,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <utility>
 #include <vector>
 
 #include "host_stage.h"
@@ -32,6 +33,15 @@ static int checks_conversions() {
       CHECK(y[n + o] == 0xa5);
     }
   }
+  // fractions, values no int32 holds, infinities, NaN: what the device's conversion gives (-1 stands for 0x7fffffff's low byte)
+  const std::vector<std::pair<float, int>> odd = {{-0.9f, 0}, {1.9f, 1}, {-1.5f, -1}, {2147483520.f, 0x80}, {2147483648.f, -1}, {3e9f, -1}, {INFINITY, -1},
+                                                  {-2147483648.f, 0}, {-3e9f, 0}, {-INFINITY, 0}, {NAN, 0}, {300.f, 44}, {-129.f, 127}};
+  std::vector<float> of;
+  for (int r = 0; r < 5; ++r)
+    for (auto& v : odd) of.push_back(v.first);
+  std::vector<uint8_t> ob(of.size());
+  host_f32_to_bytes(of.data(), ob.data(), of.size());
+  for (size_t i = 0; i < of.size(); ++i) CHECK(ob[i] == (uint8_t)odd[i % odd.size()].second);
   for (int dt : {B200Q_DT_I8, B200Q_DT_U8, B200Q_DT_I16, B200Q_DT_U16, B200Q_DT_I32}) {
     for (size_t n : {0, 1, 31, 32, 33, 257}) {
       std::vector<int32_t> raw(n + 8);

@@ -12,8 +12,11 @@
 namespace b200q {
 namespace {
 
+// the low byte of x as an int32, out of range to the nearest end and NaN to 0, as the GPU converts
+uint8_t f32_low_byte(float x) { return x >= 2147483648.f ? 0xff : (x >= -2147483648.f ? (uint8_t)(int)x : 0); }
+
 void f32_to_bytes_scalar(const float* x, uint8_t* y, size_t n) {
-  for (size_t i = 0; i < n; ++i) y[i] = (uint8_t)(int)x[i];
+  for (size_t i = 0; i < n; ++i) y[i] = f32_low_byte(x[i]);
 }
 
 template <typename T>
@@ -22,15 +25,18 @@ void q_to_f32_scalar(const T* x, float* y, size_t n) {
 }
 
 #ifdef B200Q_HOST_AVX2
+// cvttps gives 0x80000000 for what does not fit; above the range the low byte has to be that of 0x7fffffff
+__attribute__((target("avx2"))) inline __m256i low_bytes(const float* x) {
+  const __m256 v = _mm256_loadu_ps(x);
+  const __m256i above = _mm256_castps_si256(_mm256_cmp_ps(v, _mm256_set1_ps(2147483648.f), _CMP_GE_OQ));
+  return _mm256_and_si256(_mm256_or_si256(_mm256_cvttps_epi32(v), above), _mm256_set1_epi32(0xff));
+}
+
 __attribute__((target("avx2"))) void f32_to_bytes_avx2(const float* x, uint8_t* y, size_t n) {
-  const __m256i low = _mm256_set1_epi32(0xff);
   const __m256i order = _mm256_setr_epi32(0, 4, 1, 5, 2, 6, 3, 7);   // undo the per-128-bit-lane packing
   size_t i = 0;
   for (; i + 32 <= n; i += 32) {
-    const __m256i a = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i)), low);
-    const __m256i b = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i + 8)), low);
-    const __m256i c = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i + 16)), low);
-    const __m256i d = _mm256_and_si256(_mm256_cvttps_epi32(_mm256_loadu_ps(x + i + 24)), low);
+    const __m256i a = low_bytes(x + i), b = low_bytes(x + i + 8), c = low_bytes(x + i + 16), d = low_bytes(x + i + 24);
     const __m256i p = _mm256_packus_epi16(_mm256_packus_epi32(a, b), _mm256_packus_epi32(c, d));
     _mm256_storeu_si256(reinterpret_cast<__m256i*>(y + i), _mm256_permutevar8x32_epi32(p, order));
   }
