@@ -1,12 +1,16 @@
 // The operator face's host side (csrc/host_stage.cpp, csrc/host_convert.cpp) on host memory, without a device: the CUDA calls it
 // makes are the fakes below, which work at once and can be told to fail.  usage: host_stage_check <check>
 #include <cuda_runtime.h>
+#include <dlfcn.h>
+#include <errno.h>
 #include <math.h>
-#include <stdarg.h>
+#include <pthread.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
+#include <new>
 #include <utility>
 #include <vector>
 
@@ -21,6 +25,131 @@ using namespace b200q;
       exit(1);                                                         \
     }                                                                  \
   } while (0)
+
+// ------------------------------------------------------------------------------------------------ fakes
+namespace fake {
+int streams_made, streams_ended, events_made, events_ended, memory_made, memory_ended, threads_made;
+int fail_stream = -1, fail_copy = -1;   // which call fails (counted from 0), -1: none
+int threads_allowed = 1 << 30;
+bool null_stream_used;
+int copies;
+std::mutex m;
+}  // namespace fake
+
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { std::lock_guard<std::mutex> l(fake::m); ++fake::memory_made; *p = malloc(n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { std::lock_guard<std::mutex> l(fake::m); ++fake::memory_ended; free(p); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { std::lock_guard<std::mutex> l(fake::m); ++fake::memory_made; *p = malloc(n); memset(*p, 0xee, n); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { std::lock_guard<std::mutex> l(fake::m); ++fake::memory_ended; free(p); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
+  std::lock_guard<std::mutex> l(fake::m);
+  if (fake::fail_stream >= 0 && fake::fail_stream-- == 0) return cudaErrorMemoryAllocation;
+  ++fake::streams_made;
+  *s = reinterpret_cast<cudaStream_t>(malloc(1));
+  return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t s) { std::lock_guard<std::mutex> l(fake::m); ++fake::streams_ended; free(s); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { std::lock_guard<std::mutex> l(fake::m); ++fake::events_made; *e = reinterpret_cast<cudaEvent_t>(malloc(1)); return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { std::lock_guard<std::mutex> l(fake::m); ++fake::events_ended; free(e); return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) { memset(p, v, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {
+  std::lock_guard<std::mutex> l(fake::m);
+  ++fake::copies;
+  if (st == nullptr) fake::null_stream_used = true;
+  if (fake::fail_copy >= 0 && fake::fail_copy-- == 0) return cudaErrorUnknown;
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
+const char* cudaGetErrorString(cudaError_t) { return "fake"; }
+cudaError_t cudaGetLastError() { return cudaErrorUnknown; }
+// (the program's own definition comes before the C library's for the C++ runtime too)
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* arg) {
+  typedef int (*create_t)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+  static create_t real = reinterpret_cast<create_t>(dlsym(RTLD_NEXT, "pthread_create"));
+  if (fake::threads_made >= fake::threads_allowed) return EAGAIN;
+  ++fake::threads_made;
+  return real(t, a, f, arg);
+}
+}
+
+// the n-th request for memory from now on fails, once
+static std::atomic<int> new_fails{-1};
+void* operator new(size_t n) {
+  if (new_fails.load() >= 0 && new_fails.fetch_sub(1) == 0) throw std::bad_alloc();
+  if (void* p = malloc(n ? n : 1)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { free(p); }
+void operator delete(void* p, size_t) noexcept { free(p); }
+
+namespace b200q {
+int set_error(int code, const char*, ...) { return code; }
+int cuda_error(cudaError_t e, const char*, const char*, int) { return e == cudaErrorMemoryAllocation ? B200Q_ERR_NOMEM : B200Q_ERR_CUDA; }
+}  // namespace b200q
+
+// ------------------------------------------------------------------------------------------------ checks
+// rows of K bytes -> N values: out[n] = x[n % K] + n (as the storage type)
+static int run_rows(HostStage& stage, const float* x, float* y, int64_t rows, int K, int N, int dt) {
+  const size_t size = dt == B200Q_DT_I32 ? 4 : (dt == B200Q_DT_I16 || dt == B200Q_DT_U16 ? 2 : 1);
+  int status = 77;
+  const int rc = stage.run(x, y, rows, (size_t)K, (size_t)N, dt, size, &status, [&](int64_t, int64_t cnt, const uint8_t* xb, void* yb, int* st, cudaStream_t) {
+    CHECK(*st == 0);
+    for (int64_t r = 0; r < cnt; ++r)
+      for (int n = 0; n < N; ++n) {
+        const int v = (int8_t)xb[r * K + n % K] + n % 50;
+        if (size == 4) static_cast<int32_t*>(yb)[r * N + n] = v;
+        else if (size == 2) static_cast<int16_t*>(yb)[r * N + n] = (int16_t)v;
+        else static_cast<int8_t*>(yb)[r * N + n] = (int8_t)v;
+      }
+    return B200Q_OK;
+  });
+  if (rc == B200Q_OK) CHECK(status == 0);
+  return rc;
+}
+
+static void check_rows(HostStage& stage, int64_t rows, int K, int N, int dt, int expect = B200Q_OK) {
+  std::vector<float> x((size_t)rows * K), y((size_t)rows * N, 1e9f);
+  for (size_t i = 0; i < x.size(); ++i) x[i] = (float)((int)(i * 7 % 61) - 30);
+  CHECK(run_rows(stage, x.data(), y.data(), rows, K, N, dt) == expect);
+  if (expect != B200Q_OK) return;
+  for (int64_t r = 0; r < rows; ++r)
+    for (int n = 0; n < N; ++n) CHECK(y[(size_t)(r * N + n)] == x[(size_t)(r * K + n % K)] + (float)(n % 50));
+}
+
+static void check_shapes() {
+  HostStage stage;
+  for (int dt : {B200Q_DT_I8, B200Q_DT_I16, B200Q_DT_I32}) {
+    check_rows(stage, 3, 17, 5, dt);                    // by the calling thread
+    check_rows(stage, 300, 999, 77, dt);                // one piece, by the pool
+    check_rows(stage, 5000, 777, 33, dt);               // more pieces than slots, odd rows
+    check_rows(stage, 700, 33, 1001, dt);
+    check_rows(stage, 1, 700000, 9, dt);                // one unit larger than a piece
+  }
+}
+
+static int checks_pieces() {
+  {
+    std::vector<std::thread> t;
+    for (int i = 0; i < 3; ++i) t.emplace_back(check_shapes);
+    check_shapes();
+    for (auto& x : t) x.join();
+  }
+  CHECK(fake::streams_made > 0 && fake::streams_made == fake::streams_ended && fake::events_made == fake::events_ended && fake::memory_made == fake::memory_ended);
+  return 0;
+}
+
+// Threads that cannot be had are done without: the calling thread does their work.
+static int checks_threads(int allowed) {
+  fake::threads_allowed = allowed;
+  check_shapes();
+  CHECK(fake::threads_made <= allowed);
+  return 0;
+}
 
 static int checks_conversions() {
   std::vector<float> f;
@@ -65,9 +194,31 @@ static int checks_conversions() {
   return 0;
 }
 
+// Every request for host memory of a call fails once: the call works, or says so and the next one works.
+static int checks_memory() {
+  std::vector<float> x(1500 * 999, 3.f), y(1500 * 77, 0.f);
+  int refused = 0, passed = 0;
+  for (int n = 0; n < 120; ++n) {
+    HostStage stage;
+    new_fails.store(n);
+    const int rc = run_rows(stage, x.data(), y.data(), 1500, 999, 77, B200Q_DT_I8);
+    const bool met = new_fails.exchange(-1) < 0;
+    CHECK(rc == B200Q_OK || rc == B200Q_ERR_NOMEM);
+    ++(rc == B200Q_OK ? passed : refused);
+    check_rows(stage, 1500, 999, 77, B200Q_DT_I8);
+    if (!met) break;   // more than the call asks for
+  }
+  CHECK(refused > 3 && passed > 3);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "conversions")) return checks_conversions();
+  if (!strcmp(what, "pieces")) return checks_pieces();
+  if (!strcmp(what, "no threads")) return checks_threads(0);
+  if (!strcmp(what, "out of memory")) return checks_memory();
+  if (!strcmp(what, "two threads")) return checks_threads(2);
   fprintf(stderr, "unknown check '%s'\n", what);
   return 2;
 }

@@ -18,7 +18,8 @@ pytestmark = pytest.mark.skipif(shutil.which("g++") is None or not os.path.exist
 def program(request, tmp_path_factory):
     out = str(tmp_path_factory.mktemp("host_stage") / "check")
     cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-Wno-unused-function", "-ffp-contract=off", "-pthread", "-I" + CSRC, "-I" + os.path.join(CUDA, "include"),
-           os.path.join(ROOT, "tests", "host_stage_check.cpp"), os.path.join(CSRC, "host_convert.cpp"), "-o", out]
+           os.path.join(ROOT, "tests", "host_stage_check.cpp"), os.path.join(CSRC, "host_convert.cpp"),
+           os.path.join(CSRC, "host_stage.cpp"), "-o", out, "-ldl"]
     if request.param == "plain":
         cmd.append("-DB200Q_PORTABLE_HOST")
     r = subprocess.run(cmd, capture_output=True, text=True)
@@ -26,7 +27,7 @@ def program(request, tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["conversions"])
+@pytest.mark.parametrize("what", ["conversions", "pieces", "no threads", "two threads", "out of memory"])
 def test_host_stage(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr

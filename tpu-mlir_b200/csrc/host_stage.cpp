@@ -12,6 +12,8 @@
 #include <sched.h>
 #include <string.h>
 
+#include <exception>
+
 namespace b200q {
 namespace {
 
@@ -46,7 +48,10 @@ void HostPool::start() {
   int cpus = 1;
   if (sched_getaffinity(0, sizeof(set), &set) == 0) cpus = CPU_COUNT(&set);
   const int workers = cpus - 1 < 15 ? cpus - 1 : 15;   // memory bandwidth is used up well before 16 cores
-  for (int i = 0; i < workers; ++i) threads_.emplace_back([this] { loop(); });
+  try {
+    for (int i = 0; i < workers; ++i) threads_.emplace_back([this] { loop(); });
+  } catch (const std::exception&) {   // no more threads to be had: a submitter helps with its own tasks anyway
+  }
 }
 
 HostPool::~HostPool() {
@@ -65,11 +70,20 @@ HostPool::~HostPool() {
 }
 
 void HostPool::submit(const HostTask* tasks, size_t n) {
+  bool queued = false;
   {
     std::lock_guard<std::mutex> lock(m_);
     if (!started_) start();
-    q_.insert(q_.end(), tasks, tasks + n);
+    try {
+      q_.insert(q_.end(), tasks, tasks + n);
+      queued = true;
+    } catch (const std::exception&) {   // (inserting at the end has no effect then)
+    }
     queued_.store((int)q_.size(), std::memory_order_relaxed);
+  }
+  if (!queued) {
+    for (size_t i = 0; i < n; ++i) tasks[i].run();
+    return;
   }
   if (n == 1) cv_.notify_one();
   else cv_.notify_all();
@@ -130,11 +144,12 @@ void HostPool::give(Pinned b) {
   if (!b.p) return;
   {
     std::lock_guard<std::mutex> lock(cache_m_);
-    if (cached_ + b.cap <= CACHE_BYTES) {
-      cache_.push_back(b);
-      cached_ += b.cap;
-      return;
-    }
+    if (cached_ + b.cap <= CACHE_BYTES) try {
+        cache_.push_back(b);
+        cached_ += b.cap;
+        return;
+      } catch (const std::exception&) {   // given back to the system instead
+      }
   }
   cudaFreeHost(b.p);
 }
@@ -156,14 +171,15 @@ int HostPool::take(Streams* out) {
   return B200Q_OK;
 }
 
-void HostPool::give(Streams st) {
+void HostPool::give(const Streams& st) {
   if (st.device < 0) return;
   {
     std::lock_guard<std::mutex> lock(cache_m_);
-    if (sets_.size() < CACHE_SETS) {
-      sets_.push_back(st);
-      return;
-    }
+    if (sets_.size() < CACHE_SETS) try {
+        sets_.push_back(st);
+        return;
+      } catch (const std::exception&) {
+      }
   }
   for (auto& e : st.ev) cudaEventDestroy(e);
   for (auto& x : st.s)
@@ -194,6 +210,7 @@ void HostStage::convert(const void* src, void* dst, size_t n, int dt, size_t out
   }
   const size_t step = TASK_VALUES / 4, ss = dt < 0 ? 4 : out_size, ds = dt < 0 ? 1 : 4;
   std::vector<HostTask> tasks;
+  tasks.reserve((n + step - 1) / step);
   std::atomic<int> left{(int)((n + step - 1) / step)};
   for (size_t o = 0; o < n; o += step)
     tasks.push_back(HostTask{static_cast<const uint8_t*>(src) + o * ss, static_cast<uint8_t*>(dst) + o * ds, n - o < step ? n - o : step, dt, &left, past_cache});
@@ -204,6 +221,16 @@ void HostStage::convert(const void* src, void* dst, size_t n, int dt, size_t out
 
 int HostStage::run(const float* x, float* y, int64_t units, size_t x_per, size_t y_per, int out_dt, size_t out_size, int* status,
                    const Launch& launch) {
+  try {   // the callers are C entries.  Nothing is in flight where memory is asked for.
+    return run_checked(x, y, units, x_per, y_per, out_dt, out_size, status, launch);
+  } catch (const std::exception& e) {
+    status_at_ = ~size_t(0);
+    return set_error(B200Q_ERR_NOMEM, "operator face: %s", e.what());
+  }
+}
+
+int HostStage::run_checked(const float* x, float* y, int64_t units, size_t x_per, size_t y_per, int out_dt, size_t out_size, int* status,
+                           const Launch& launch) {
   if (!pool_) pool_ = HostPool::get();
   const size_t larger = x_per > y_per ? x_per : y_per;
   const size_t x_total = x_per * (size_t)units, y_bytes = y_per * (size_t)units * out_size;
@@ -254,6 +281,7 @@ int HostStage::run_pieces(const float* x, float* y, int64_t units, int64_t per, 
   B200Q_TRY(grow(&in_, xs * slots));
   B200Q_TRY(grow(&out_, ys * slots + 16));
   if (streams_.device < 0) B200Q_TRY(pool_->take(&streams_));
+  streams_.ev.reserve(3 * MAX_SLOTS);
   while ((int)streams_.ev.size() < 3 * slots) {
     cudaEvent_t e;
     CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -268,6 +296,7 @@ int HostStage::run_pieces(const float* x, float* y, int64_t units, int64_t per, 
   auto count = [&](int c) { return first(c) + per <= units ? per : units - first(c); };
   const bool past_cache = y_per * (size_t)units >= PAST_CACHE_VALUES;
   std::vector<HostTask> tasks;
+  tasks.reserve(((size_t)per * (x_per > y_per ? x_per : y_per) + TASK_VALUES - 1) / TASK_VALUES);   // nothing below asks for memory
   auto submit = [&](const void* src, void* dst, size_t n, int dt, std::atomic<int>* left) {
     const size_t ss = dt < 0 ? 4 : out_size, ds = dt < 0 ? 1 : 4;
     tasks.clear();
@@ -306,7 +335,11 @@ int HostStage::run_pieces(const float* x, float* y, int64_t units, int64_t per, 
       chk(cudaMemcpyAsync(x_dev_.as<uint8_t>() + xo, in_.p + xs * (size_t)slot, xn, cudaMemcpyHostToDevice, s_in), "H2D input");
       chk(cudaEventRecord(ev(0, slot), s_in), "event");
       chk(cudaStreamWaitEvent(s_cmp, ev(0, slot), 0), "event");
-      if (rc == B200Q_OK) rc = launch(first(c), count(c), x_dev_.as<uint8_t>() + xo, y_dev_.as<uint8_t>() + yo, status_dev, s_cmp);
+      try {
+        if (rc == B200Q_OK) rc = launch(first(c), count(c), x_dev_.as<uint8_t>() + xo, y_dev_.as<uint8_t>() + yo, status_dev, s_cmp);
+      } catch (const std::exception& e) {   // (pieces are in flight: this function ends by waiting for them)
+        rc = set_error(B200Q_ERR_NOMEM, "operator face: %s", e.what());
+      }
       chk(cudaEventRecord(ev(1, slot), s_cmp), "event");
       chk(cudaStreamWaitEvent(s_out, ev(1, slot), 0), "event");
       chk(cudaMemcpyAsync(out_.p + ys * (size_t)slot, y_dev_.as<uint8_t>() + yo, yn, cudaMemcpyDeviceToHost, s_out), "D2H output");

@@ -8,7 +8,6 @@
 #include <atomic>
 #include <condition_variable>
 #include <deque>
-#include <functional>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -58,7 +57,7 @@ class HostPool {
   int take(size_t bytes, Pinned* out);
   void give(Pinned b);
   int take(Streams* out);
-  void give(Streams st);
+  void give(const Streams& st);
 
  private:
   static constexpr size_t CACHE_BYTES = 64u << 20, CACHE_SETS = 8;
@@ -85,10 +84,23 @@ class HostStage {
   // piece of units launch(first, count, x_dev, y_dev, status_dev, stream) enqueues the kernels.  status_dev is an int
   // that is zero before the call and comes back with the results in *status.  Synchronous; everything the caller
   // queued on the default stream is finished before the first kernel.
-  typedef std::function<int(int64_t, int64_t, const uint8_t*, void*, int*, cudaStream_t)> Launch;
+  // (refers to the caller's function object: making it asks for no memory)
+  class Launch {
+   public:
+    template <typename F>
+    Launch(const F& f) : object_(&f), call_([](const void* o, int64_t first, int64_t n, const uint8_t* x, void* y, int* st, cudaStream_t s) -> int {
+      return (*static_cast<const F*>(o))(first, n, x, y, st, s);
+    }) {}
+    int operator()(int64_t first, int64_t n, const uint8_t* x, void* y, int* st, cudaStream_t s) const { return call_(object_, first, n, x, y, st, s); }
+
+   private:
+    const void* object_;
+    int (*call_)(const void*, int64_t, int64_t, const uint8_t*, void*, int*, cudaStream_t);
+  };
   int run(const float* x, float* y, int64_t units, size_t x_per, size_t y_per, int out_dt, size_t out_size, int* status, const Launch& launch);
 
  private:
+  int run_checked(const float* x, float* y, int64_t units, size_t x_per, size_t y_per, int out_dt, size_t out_size, int* status, const Launch& launch);
   int grow(HostPool::Pinned* b, size_t bytes);
   int run_pieces(const float* x, float* y, int64_t units, int64_t per, size_t x_per, size_t y_per, int out_dt, size_t out_size, int* status,
                  const Launch& launch);
