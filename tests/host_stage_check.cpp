@@ -212,11 +212,43 @@ static int checks_memory() {
   return 0;
 }
 
+// A stream that cannot be made: the call fails, nothing half-made is kept, and the next call has three streams again.
+static int checks_streams() {
+  for (int n = 0; n < 3; ++n) {
+    HostStage stage, other;
+    fake::fail_stream = n;
+    check_rows(stage, 1500, 999, 77, B200Q_DT_I8, B200Q_ERR_NOMEM);
+    CHECK(fake::streams_made == fake::streams_ended);
+    fake::null_stream_used = false;
+    check_rows(stage, 1500, 999, 77, B200Q_DT_I8);
+    check_rows(other, 1500, 999, 77, B200Q_DT_I8);
+    CHECK(!fake::null_stream_used);
+  }
+  return 0;
+}
+
+// A copy that fails, early or late: the call says so and the next one is right.
+static int checks_copies() {
+  HostStage stage;
+  fake::copies = 0;
+  check_rows(stage, 1500, 999, 77, B200Q_DT_I8);
+  const int copies = fake::copies;
+  for (int n = 0; n < copies; ++n) {
+    fake::fail_copy = n;
+    check_rows(stage, 1500, 999, 77, B200Q_DT_I8, B200Q_ERR_CUDA);
+    fake::fail_copy = -1;
+    check_rows(stage, 1500, 999, 77, B200Q_DT_I8);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "conversions")) return checks_conversions();
   if (!strcmp(what, "pieces")) return checks_pieces();
   if (!strcmp(what, "no threads")) return checks_threads(0);
+  if (!strcmp(what, "streams")) return checks_streams();
+  if (!strcmp(what, "copies")) return checks_copies();
   if (!strcmp(what, "out of memory")) return checks_memory();
   if (!strcmp(what, "two threads")) return checks_threads(2);
   fprintf(stderr, "unknown check '%s'\n", what);

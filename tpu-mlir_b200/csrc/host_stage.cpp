@@ -166,8 +166,17 @@ int HostPool::take(Streams* out) {
         return B200Q_OK;
       }
   }
-  out->device = dev;
-  for (auto& st : out->s) CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  Streams made;
+  for (auto& st : made.s) {
+    const cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) continue;
+    st = nullptr;
+    for (auto& x : made.s)
+      if (x) cudaStreamDestroy(x);
+    return cuda_error(e, "cudaStreamCreateWithFlags", __FILE__, __LINE__);
+  }
+  made.device = dev;
+  *out = made;
   return B200Q_OK;
 }
 
