@@ -242,6 +242,24 @@ static int checks_copies() {
   return 0;
 }
 
+// A result that is written over its own input (rows grow in place, or shrink).
+static int checks_overlap() {
+  const int64_t rows = 4000;
+  for (int N : {999, 501, 333}) {
+    const int K = N == 333 ? 999 : 500;
+    for (int64_t shift : {int64_t(0), int64_t(12345)}) {   // of the result within the buffer
+      HostStage stage;
+      std::vector<float> buf((size_t)rows * 1000 + 20000), want((size_t)rows * N);
+      for (size_t i = 0; i < buf.size(); ++i) buf[i] = (float)((int)(i * 7 % 61) - 30);
+      for (int64_t r = 0; r < rows; ++r)
+        for (int n = 0; n < N; ++n) want[(size_t)(r * N + n)] = buf[(size_t)(r * K + n % K)] + (float)(n % 50);
+      CHECK(run_rows(stage, buf.data(), buf.data() + shift, rows, K, N, B200Q_DT_I8) == B200Q_OK);
+      CHECK(!memcmp(buf.data() + shift, want.data(), want.size() * 4));
+    }
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "conversions")) return checks_conversions();
@@ -249,6 +267,7 @@ int main(int argc, char** argv) {
   if (!strcmp(what, "no threads")) return checks_threads(0);
   if (!strcmp(what, "streams")) return checks_streams();
   if (!strcmp(what, "copies")) return checks_copies();
+  if (!strcmp(what, "overlap")) return checks_overlap();
   if (!strcmp(what, "out of memory")) return checks_memory();
   if (!strcmp(what, "two threads")) return checks_threads(2);
   fprintf(stderr, "unknown check '%s'\n", what);

@@ -244,6 +244,10 @@ int HostStage::run_checked(const float* x, float* y, int64_t units, size_t x_per
   const size_t larger = x_per > y_per ? x_per : y_per;
   const size_t x_total = x_per * (size_t)units, y_bytes = y_per * (size_t)units * out_size;
   int64_t per = (int64_t)((PIECE_VALUES + larger - 1) / larger);
+  // a result that lies over its input is written when all of the input has been read
+  if (reinterpret_cast<uintptr_t>(x) < reinterpret_cast<uintptr_t>(y + y_per * (size_t)units) &&
+      reinterpret_cast<uintptr_t>(y) < reinterpret_cast<uintptr_t>(x + x_total))
+    per = units;
   if (per > units) per = units;
   const bool single = per == units;
   cudaStream_t s = 0;
