@@ -14,6 +14,7 @@
 #include <utility>
 #include <vector>
 
+#include "held_array.h"
 #include "host_stage.h"
 
 using namespace b200q;
@@ -260,6 +261,31 @@ static int checks_overlap() {
   return 0;
 }
 
+// An upload that fails: the next call does not take the old contents, or half of the new, for what is on the device.
+static int checks_held_arrays() {
+  HeldArray mult, shift;
+  const std::vector<int32_t> m1 = {1, 2, 3}, s1 = {4, 5, 6}, m2 = {7, 8, 9}, s2 = {9, 9, 9};
+  auto both = [&](const std::vector<int32_t>& m, const std::vector<int32_t>& s) {
+    const int rc = mult.put(m, nullptr);
+    return rc != B200Q_OK ? rc : shift.put(s, nullptr);
+  };
+  auto holds = [&](const std::vector<int32_t>& m, const std::vector<int32_t>& s) {
+    return !memcmp(mult.get(), m.data(), m.size() * 4) && !memcmp(shift.get(), s.data(), s.size() * 4);
+  };
+  CHECK(both(m1, s1) == B200Q_OK && holds(m1, s1));
+  fake::copies = 0;
+  CHECK(both(m1, s1) == B200Q_OK && fake::copies == 0);
+  for (int n = 0; n < 2; ++n) {
+    fake::fail_copy = n;
+    CHECK(both(m2, s2) == B200Q_ERR_CUDA);
+    fake::fail_copy = -1;
+    CHECK(both(m1, s1) == B200Q_OK && holds(m1, s1));
+  }
+  CHECK(both(m2, s1) == B200Q_OK && holds(m2, s1));
+  CHECK(both({1}, {2, 3, 4, 5}) == B200Q_OK && holds({1}, {2, 3, 4, 5}));
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "conversions")) return checks_conversions();
@@ -268,6 +294,7 @@ int main(int argc, char** argv) {
   if (!strcmp(what, "streams")) return checks_streams();
   if (!strcmp(what, "copies")) return checks_copies();
   if (!strcmp(what, "overlap")) return checks_overlap();
+  if (!strcmp(what, "held arrays")) return checks_held_arrays();
   if (!strcmp(what, "out of memory")) return checks_memory();
   if (!strcmp(what, "two threads")) return checks_threads(2);
   fprintf(stderr, "unknown check '%s'\n", what);

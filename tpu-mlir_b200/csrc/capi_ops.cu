@@ -9,6 +9,7 @@
 
 #include "devbuf.h"
 #include "eltwise.h"
+#include "held_array.h"
 #include "host_stage.h"
 #include "igemm.h"
 #include "internal.h"
@@ -46,9 +47,7 @@ struct ResolvedRequant {
   std::vector<int32_t> multiplier, shift;
 };
 
-// `cached` (optional): the arrays d_mult / d_shift hold from an earlier call; equal ones are not uploaded again.
-int make_epilogue(const ResolvedRequant& r, const int32_t* d_bias, DevBuf& d_mult, DevBuf& d_shift, cudaStream_t s,
-                  Epilogue* e, ResolvedRequant* cached = nullptr) {
+int make_epilogue(const ResolvedRequant& r, const int32_t* d_bias, HeldArray& d_mult, HeldArray& d_shift, cudaStream_t s, Epilogue* e) {
   e->dialect = r.dialect;
   e->round_mode = r.round_mode;
   e->per_channel = r.per_channel;
@@ -60,14 +59,13 @@ int make_epilogue(const ResolvedRequant& r, const int32_t* d_bias, DevBuf& d_mul
   e->multiplier = nullptr;
   e->shift = nullptr;
   if (!r.multiplier.empty()) {
-    if (!cached || cached->multiplier != r.multiplier) B200Q_TRY(d_mult.upload(r.multiplier.data(), r.multiplier.size() * 4, s));
-    e->multiplier = d_mult.as<int32_t>();
+    B200Q_TRY(d_mult.put(r.multiplier, s));
+    e->multiplier = d_mult.get();
   }
   if (!r.shift.empty()) {
-    if (!cached || cached->shift != r.shift) B200Q_TRY(d_shift.upload(r.shift.data(), r.shift.size() * 4, s));
-    e->shift = d_shift.as<int32_t>();
+    B200Q_TRY(d_shift.put(r.shift, s));
+    e->shift = d_shift.get();
   }
-  if (cached) *cached = r;
   return B200Q_OK;
 }
 
@@ -196,9 +194,9 @@ int gemm_dispatch(const void* a, int a_dt, const void* b_nk, int b_dt, int64_t M
 }
 
 struct MatMulHandle {
-  DevBuf stage_f32, a_q8, b_f32, b_nk, bias, mult, shift, out_q, out_f32, status, perm;
+  DevBuf stage_f32, a_q8, b_f32, b_nk, bias, out_q, out_f32, status, perm;
+  HeldArray mult, shift;
   HostStage host;
-  ResolvedRequant requant;   // what mult / shift hold
   bool weights_ready = false;
   int weight_version = -1;
   const float* weight_ptr = nullptr;
@@ -251,7 +249,8 @@ struct ConvHandle {
   int kpad = 0;             // im2col row length (KH*KW*IC rounded up to 16)
   int bh = 0, bw = 0, Hp = 0, Wp = 0;
   Epilogue epi{};
-  DevBuf w_oihw, w_packed, bias, mult, shift, x_bordered, a_cols, status;
+  DevBuf w_oihw, w_packed, bias, x_bordered, a_cols, status;
+  HeldArray mult, shift;
   // operator-face staging
   DevBuf w_f32, bias_f32;
   HostStage host;   // host copies pipelined over pieces of the batch
@@ -650,7 +649,7 @@ int b200q_matmul_inference(const b200q_matmul_desc* desc, float* const* inputs, 
       ResolvedRequant r;
       Epilogue e;
       if ((rc = resolve_matmul(d, multi_f, 0, &r))) break;
-      if ((rc = make_epilogue(r, bias_f ? h->bias.as<int32_t>() : nullptr, h->mult, h->shift, s, &e, &h->requant))) break;
+      if ((rc = make_epilogue(r, bias_f ? h->bias.as<int32_t>() : nullptr, h->mult, h->shift, s, &e))) break;
       int status = 0;
       rc = h->host.run(inputs[0], outputs[0], rows, (size_t)d.K, (size_t)d.N, d.out_dtype, dtype_size(d.out_dtype), &status,
                        [&](int64_t, int64_t cnt, const uint8_t* x, void* y, int* st_dev, cudaStream_t st) {
@@ -662,7 +661,6 @@ int b200q_matmul_inference(const b200q_matmul_desc* desc, float* const* inputs, 
     }
     if ((rc = h->status.ensure(4))) break;
     if (cudaMemsetAsync(h->status.p, 0, 4, s) != cudaSuccess) { rc = cuda_error(cudaGetLastError(), "memset", __FILE__, __LINE__); break; }
-    h->requant = ResolvedRequant();   // the arrays below are uploaded once per batch entry
     if ((rc = h->stage_f32.ensure(a_elems * 4 > (size_t)d.N * 4 ? a_elems * 4 : (size_t)d.N * 4))) break;
     if ((rc = h->a_q8.ensure(a_elems))) break;
     if ((rc = h->out_q.ensure(o_elems * dtype_size(d.out_dtype)))) break;
@@ -687,7 +685,7 @@ int b200q_matmul_inference(const b200q_matmul_desc* desc, float* const* inputs, 
       ResolvedRequant r;
       if ((rc = resolve_matmul(d, multi_f, b, &r))) break;
       Epilogue e;
-      // per-launch multiplier/shift arrays: small, re-uploaded (stream ordered) for each batch entry
+      // per-launch multiplier/shift arrays: small, uploaded again (stream ordered) where a batch entry's differ
       if ((rc = make_epilogue(r, bias_f ? h->bias.as<int32_t>() : nullptr, h->mult, h->shift, s, &e))) break;
       const uint8_t* a = h->a_q8.as<uint8_t>() + (size_t)b * d.M * d.K;
       const uint8_t* bm = h->b_nk.as<uint8_t>() + (d.right_batched ? (size_t)b * d.K * d.N : 0);
