@@ -61,6 +61,28 @@ def test_single_pass_equals_two_passes(m):
     assert all(np.array_equal(one._shard[k], two._shard[k]) for k in ("minmax", "hist", "sizes"))
 
 
+@pytest.mark.parametrize("shape", [(3, 40), (5, 40), (8, 10), (2,), ()])
+def test_activations_that_are_not_the_batch_are_refused(m, shape):
+    """Cut at the first tensor's batch they would count as other samples, or lose their tail: every driver refuses them."""
+    bad = torch.ones(shape, device="cuda")
+    for kw in ({}, dict(cache_bytes=1 << 30), dict(cache_bytes=0)):
+        cal = ShardedCalibrator(lambda b: {"a": torch.ones((4, 10), device="cuda"), "bad": bad}, math=m)
+        with pytest.raises((ValueError, RuntimeError, IndexError)):
+            cal.run([0], 4, **kw)
+
+
+def test_an_activation_that_is_the_same_in_every_sample(m):
+    """One row for the whole batch (a position table, say) counts once per sample, as in the driver that keeps the activations."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    a, one = torch.randn((4, 100), device="cuda", generator=g), torch.randn((1, 30), device="cuda", generator=g)
+    res = []
+    for kw in ({}, dict(cache_bytes=1 << 30)):
+        cal = ShardedCalibrator(lambda b: {"a": a * b, "one": one}, math=m)
+        res.append((cal.run([1.0, 2.0], 8, **kw), cal.histograms["one"].cpu()))
+    assert res[0][0] == res[1][0] and torch.equal(res[0][1], res[1][1]) and int(res[0][1].sum()) == 8 * 30
+
+
 @pytest.mark.parametrize("bins", [128, 256, 2049, 5000, 45000, 131072, 300001])
 def test_kld_of_long_and_sparse_histograms(m, bins):
     rng = np.random.default_rng(bins)

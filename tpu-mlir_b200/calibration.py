@@ -469,6 +469,15 @@ class ShardedCalibrator:
         return out
 
 
+    @staticmethod
+    def _samples(name, x, B):
+        """The activation as a tensor of B samples: its first dimension is B, or 1 for what is the same in every sample."""
+        if x.dim() and x.shape[0] == B:
+            return x
+        if x.dim() and x.shape[0] == 1:
+            return x.expand((B,) + tuple(x.shape[1:])).contiguous()
+        raise ValueError(f"{name}: the first dimension of {tuple(x.shape)} is not the batch ({B})")
+
     def _run_streaming(self, batches: Iterable, samples: int) -> Dict[str, TensorResult]:
         """One pass: per batch the forward, ONE min/max launch over all its activations, the bin schedule of its samples on
         the host (native code, one small copy back), ONE histogram launch over the activations where they lie.  Against
@@ -518,8 +527,8 @@ class ShardedCalibrator:
             if not names:
                 names = list(acts.keys())
                 sched = BinScheduler(len(names), self.bin_num)
-            xs = [m._dev(acts[n]) for n in names]
-            B = xs[0].shape[0]
+            B = acts[names[0]].shape[0]
+            xs = [self._samples(n, m._dev(acts[n]), B) for n in names]
             held += sum(x.numel() for x in xs) * 4
             mm = m.minmax_many(xs, B)
             minmax.append(mm)
