@@ -286,6 +286,15 @@ static int checks_held_arrays() {
   return 0;
 }
 
+static int checks_workers() {
+  CHECK(host_workers(16, nullptr, nullptr) == 15 && host_workers(200, nullptr, "max 100000") == 15 && host_workers(8, "", "") == 7);
+  CHECK(host_workers(1, nullptr, nullptr) == 0 && host_workers(0, nullptr, nullptr) == 0);
+  CHECK(host_workers(128, "8", nullptr) == 15 && host_workers(64, "8", nullptr) == 7 && host_workers(4, "8", nullptr) == 0 && host_workers(16, "x", nullptr) == 15);
+  CHECK(host_workers(64, nullptr, "400000 100000") == 3 && host_workers(64, nullptr, "50000 100000") == 0 && host_workers(2, nullptr, "900000 100000") == 1);
+  CHECK(host_workers(64, "2", "800000 100000") == 3);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "conversions")) return checks_conversions();
@@ -295,6 +304,7 @@ int main(int argc, char** argv) {
   if (!strcmp(what, "copies")) return checks_copies();
   if (!strcmp(what, "overlap")) return checks_overlap();
   if (!strcmp(what, "held arrays")) return checks_held_arrays();
+  if (!strcmp(what, "workers")) return checks_workers();
   if (!strcmp(what, "out of memory")) return checks_memory();
   if (!strcmp(what, "two threads")) return checks_threads(2);
   fprintf(stderr, "unknown check '%s'\n", what);

@@ -27,7 +27,7 @@ def program(request, tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["conversions", "pieces", "no threads", "two threads", "out of memory", "streams", "copies", "overlap", "held arrays"])
+@pytest.mark.parametrize("what", ["conversions", "pieces", "no threads", "two threads", "out of memory", "streams", "copies", "overlap", "held arrays", "workers"])
 def test_host_stage(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr

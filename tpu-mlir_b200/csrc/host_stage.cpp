@@ -10,6 +10,8 @@
 #include "host_stage.h"
 
 #include <sched.h>
+#include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <exception>
@@ -27,6 +29,18 @@ constexpr size_t INLINE_VALUES = 96 * 1024;      // up to here the calling threa
 constexpr size_t PAST_CACHE_VALUES = 4u << 20;
 
 }  // namespace
+
+int host_workers(int cpus, const char* local_ranks, const char* cpu_max) {
+  long long quota = 0, period = 0;
+  if (cpu_max && sscanf(cpu_max, "%lld %lld", &quota, &period) == 2 && quota > 0 && period > 0) {
+    const long long granted = (quota + period - 1) / period;
+    if (granted < cpus) cpus = (int)granted;
+  }
+  const int ranks = local_ranks ? atoi(local_ranks) : 1;
+  if (ranks > 1) cpus /= ranks;
+  const int workers = cpus - 1;                   // the calling thread is one more
+  return workers < 0 ? 0 : (workers < 15 ? workers : 15);   // memory bandwidth is used up well before 16 cores
+}
 
 // ---------------------------------------------------------------------------------------------- HostPool
 std::shared_ptr<HostPool> HostPool::get() {
@@ -47,7 +61,12 @@ void HostPool::start() {
   CPU_ZERO(&set);
   int cpus = 1;
   if (sched_getaffinity(0, sizeof(set), &set) == 0) cpus = CPU_COUNT(&set);
-  const int workers = cpus - 1 < 15 ? cpus - 1 : 15;   // memory bandwidth is used up well before 16 cores
+  char cpu_max[64] = "max";
+  if (FILE* f = fopen("/sys/fs/cgroup/cpu.max", "r")) {
+    if (!fgets(cpu_max, sizeof(cpu_max), f)) cpu_max[0] = 0;
+    fclose(f);
+  }
+  const int workers = host_workers(cpus, getenv("LOCAL_WORLD_SIZE"), cpu_max);
   try {
     for (int i = 0; i < workers; ++i) threads_.emplace_back([this] { loop(); });
   } catch (const std::exception&) {   // no more threads to be had: a submitter helps with its own tasks anyway

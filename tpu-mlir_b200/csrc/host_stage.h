@@ -34,6 +34,10 @@ struct HostTask {
   }
 };
 
+// Worker threads for a process that may run on `cpus` processors, one of `local_ranks` processes like it on the machine (as the
+// launcher says; null or nonsense: one), with a control group's quota (cpu.max: "<us> <period us>", "max ...", null: none).
+int host_workers(int cpus, const char* local_ranks, const char* cpu_max);
+
 // What the handles that stage host buffers share: worker threads (started by the first call that is large enough for
 // them), pinned memory and stream sets that a destroyed handle gave back (pinning pages and creating streams takes
 // milliseconds).  Made by the first such handle, torn down with the last one; at most CACHE_BYTES of pinned memory and
