@@ -388,7 +388,7 @@ def kernel_lines(workload, steps, warmup, a16_m=(1, 2, 4, 8, 16, 32, 128, 2048))
                                             peak_basis=f"{peaks['source']} copy bandwidth (read-only kernel)")))
     elif workload == "top":
         # fp32 Top-dialect forward (calibration's float graph): one 3x3 convolution and the whole ResNet-50 forward.
-        # The bound is the CUDA cores' fp32 FMA rate: SMs x 128 lanes x 2 flop x the SM clock sampled during the run.
+        # The bound is the tensor pipe: a product of two floats in three bf16 parts each is eight bf16 products.
         from tpu_mlir_b200 import resnet50
         n, ic, hw, oc = 64, 128, 28, 128
         x = torch.randn(n, ic, hw, hw, device="cuda")
@@ -408,23 +408,21 @@ def kernel_lines(workload, steps, warmup, a16_m=(1, 2, 4, 8, 16, 32, 128, 2048))
         xb = torch.randn(64, 3, 224, 224, device="cuda")
         mean_f = _time_steps(lambda i: fwd(xb), 10, 3)
         clocks = sampler.stop()
-        sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-        mhz = float(clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 1965.0)
-        peak = sms * 128 * 2 * mhz * 1e6 / 1e12
+        peak = peaks["bf16_tflops"] / 8
         tf_c = 2.0 * n * oc * hw * hw * ic * 9 / (mean_c * 1e-3) / 1e12
         flop_img = sum(2.0 * np.prod(fwd.shape[o["name"]]) * np.prod(o["w"].shape[1:]) for o in ops if o["type"] == "conv")
         tf_f = 64 * flop_img / (mean_f * 1e-3) / 1e12
-        basis = f"{sms} SMs x 128 fp32 lanes x 2 flop x {mhz:.0f} MHz (median SM clock sampled during the run)"
+        basis = f"{peaks['source']} bf16 GEMM rate / 8 bf16 products per fp32 product"
         lines.append(dict(metric="fp32 conv TFLOP/s", value=tf_c, unit="TFLOP/s", ms_per_step=mean_c, dtype="f32", clocks=clocks,
                           config=dict(workload="top.Conv fp32 NCHW n64 c128 28x28 oc128 k3 s1 p1 relu (ResNet-50 layer2)",
-                                      l2="input 25.7 MB + output 25.7 MB, L2-resident: the kernel is FMA-bound"),
-                          roofline=dict(bound="fp32 fma", achieved=tf_c, peak=peak, unit="TFLOP/s", frac=tf_c / peak, traffic=None,
+                                      l2="input 25.7 MB + output 25.7 MB, L2-resident: the kernel is tensor-bound"),
+                          roofline=dict(bound="tensor, 8 bf16 products per fp32 product", achieved=tf_c, peak=peak, unit="TFLOP/s", frac=tf_c / peak, traffic=None,
                                         peak_basis=basis)))
         lines.append(dict(metric="ResNet-50 fp32 forward img/s", value=64 / (mean_f * 1e-3), unit="img/s", ms_per_step=mean_f,
                           steps=10, dtype="f32",
                           config=dict(workload="ResNet-50 fp32 Top-dialect forward, batch 64, every activation kept (the calibration "
                                                "forward): 53 convolutions, pooling, adds, fc on this library's kernels"),
-                          roofline=dict(bound="fp32 fma", achieved=tf_f, peak=peak, unit="TFLOP/s", frac=tf_f / peak, traffic=None,
+                          roofline=dict(bound="tensor, 8 bf16 products per fp32 product", achieved=tf_f, peak=peak, unit="TFLOP/s", frac=tf_f / peak, traffic=None,
                                         peak_basis=basis)))
     elif workload == "peak":
         lines.append(dict(metric="tensor-pipe peak", **tensor_peaks()))

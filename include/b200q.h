@@ -499,7 +499,12 @@ typedef struct {
  * outputs[0] [n, oc, oh, ow].  Full fp32 products and sums on the CUDA cores (no tf32). */
 int b200q_top_conv2d_inference(const b200q_top_conv_desc *desc, float *const *inputs, int n_inputs,
                                float *const *outputs, int n_outputs);
-/* Device face: the handle keeps a transposed copy of the filter; `bias` stays the caller's.  run() takes any batch. */
+/* Device face: the handle keeps a transposed copy of the filter; `bias` stays the caller's.  run() takes any batch.  Without
+ * groups and from 32 channels on both sides on, products run on the tensor cores: every operand as the sum of three bf16 numbers,
+ * eight of the nine partial products (the ninth is below 2^-30 of the product) in fp32 accumulators of at most 64 products, which
+ * cut off instead of rounding, and fp32 sums over those.  Sums that are exact in fp32 are exact; the error against 64-bit sums is
+ * no larger than that of a chain of fp32 FMAs.  Infinities, NaN and what underflow may have touched are computed by FMAs.  Other
+ * convolutions are FMAs on the CUDA cores.  Scratch comes from a stream-ordered pool (allocation nodes under capture). */
 int b200q_top_conv2d_dev_create(const b200q_top_conv_desc *desc, const float *filter_oihw, const float *bias, void **handle);
 int b200q_top_conv2d_dev_run(void *handle, const float *x, float *y, int64_t batch, void *stream);
 /* Synchronises the stream and reports a kernel-side timeout, if any: the output is not valid then.  set_status names a device

@@ -297,8 +297,8 @@ class ShardedCalibrator:
         return (self.dist.get_rank(), self.dist.get_world_size()) if self.dist else (0, 1)
 
     def run(self, batches: Iterable, samples_per_rank: int, cache_bytes: Optional[int] = None) -> Dict[str, TensorResult]:
-        """``batches`` must be re-iterable (it is walked twice) and cover exactly ``samples_per_rank`` local
-        samples in order; rank r holds global samples [r*samples_per_rank, (r+1)*samples_per_rank).
+        """``batches`` must cover exactly ``samples_per_rank`` local samples in order, and be re-iterable over several ranks or
+        with ``cache_bytes`` (it may be walked twice then); rank r holds global samples [r*samples_per_rank, (r+1)*samples_per_rank).
 
         In a single process a sample's bins depend only on the samples before it, so every batch is forwarded and
         histogrammed once (``_run_streaming``) unless ``cache_bytes`` is given.  Over several ranks (or with

@@ -38,7 +38,7 @@ __global__ void nchw_to_bordered_nhwc_kernel(const uint8_t* __restrict__ x, uint
 
 
 // Fast path of the same transform for H*W % 4 == 0 and C % 4 == 0: a block moves 128 channels x 128 pixels.
-// Reads are 128-byte (512-byte for float input) coalesced runs along W, a 4x4 byte transpose happens in
+// Reads are 128-byte coalesced runs along W, a 4x4 byte transpose happens in
 // registers (prmt), the tile goes through XOR-swizzled shared memory, and writes are 128-byte runs along C.
 __device__ __forceinline__ uint32_t load4(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
 

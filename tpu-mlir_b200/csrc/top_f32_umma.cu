@@ -14,8 +14,8 @@
 // 5e-9 with an accumulator for every 16 k, which is slower); whole network 3.2e-7 against 8.0e-7.
 //
 // A k chunk of 64 costs 32 MMAs of 128 x BN x 16, an eighth of the bf16 rate: about 200 TFLOP/s of fp32 products where the
-// CUDA cores have 74.  Measured at batch 32: 3x3 128 channels 28x28 203 -> 72 us (102 TFLOP/s), 3x3 256 channels 14x14 196 ->
-// 68 us, 3x3 64 channels 56x56 285 -> 100 us, 1x1 64 to 256 channels 103 -> 52 us.  Two kernels per call:
+// CUDA cores have 74.  Measured at batch 32: 3x3 128 channels 28x28 203 -> 74 us (100 TFLOP/s), 3x3 256 channels 14x14 196 ->
+// 67 us, 3x3 64 channels 56x56 285 -> 101 us, 1x1 64 to 256 channels 103 -> 54 us.  Two kernels per call:
 //   split_f32_kernel   NCHW fp32 -> three bf16 planes [rows][channels].  Stride 1: rows are the pixels of the padded image,
 //                      and the rows of a filter tap are the same rows shifted (one TMA box per tap, no im2col).  Other
 //                      strides: rows are the output pixels, one channel run per tap.  10 bytes moved per element.

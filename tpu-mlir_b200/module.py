@@ -1069,7 +1069,8 @@ class module:  # noqa: N801  (name of the reference class)
 
     def _capture(self):
         """All ops of the graph as one CUDA graph (every launch of the device face is asynchronous on the current
-        stream and allocates nothing).  One eager pass first, so that one-time set-up is not captured."""
+        stream and allocates nothing, but for the fp32 convolutions on the tensor cores, whose scratch becomes allocation
+        nodes of the graph).  One eager pass first, so that one-time set-up is not captured."""
         torch = self.torch
         for run in self._plans:
             run()
