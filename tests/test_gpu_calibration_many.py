@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle
-from tpu_mlir_b200.calibration import CaliMathB200, ShardedCalibrator
+from tpu_mlir_b200.calibration import CaliMathB200, ShardedCalibrator, kld_threshold_host
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +92,12 @@ def test_kld_of_long_and_sparse_histograms(m, bins):
     th = m.find_thresholds([torch.from_numpy(h).cuda()], [0.01])
     hf, wf = oracle.fold_for_kld(h, np.float32(0.01), 128)
     assert th[0] == oracle.kl_diversity_hist(hf, wf, 128)
+
+
+@pytest.mark.parametrize("bins,dst", [(2048, 256), (1290, 129), (4096, 1024), (500, 500), (45000, 200), (96, 3), (66000, 264)])
+def test_kld_with_other_bin_counts(bins, dst):
+    """The C symbol takes any number of bins that divides the histogram, also more than the calibration's 128."""
+    rng = np.random.default_rng(bins)
+    h = rng.poisson(np.maximum(0.02, 400 * np.exp(-np.arange(bins) * 6 / bins))).astype(np.int32)
+    h[0] = 30_000_000
+    assert kld_threshold_host(h, np.float32(0.02), dst) == oracle.kl_diversity_hist(h, np.float32(0.02), dst)

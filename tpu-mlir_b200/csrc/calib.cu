@@ -405,12 +405,14 @@ __global__ void fold_kernel(const int* __restrict__ in, long long n_in, int* __r
 // long sums run side by side on two lanes, the bins' sums and logarithms on 32, and of the divergence itself only the
 // chain acc = (float)(acc + term) is serial (one conversion, one double addition and one conversion per non-empty bin).
 // 73 histograms of 2048 to 3000 bins: 1690 us with one thread per candidate, dominated by two log10 calls per bin in a
-// row; see the call's time in the notes of the calibration driver.
+// row, 157 us this way.
 constexpr int KLD_WARPS = 16;
 constexpr int KLD_SMEM_BINS = 40 * 1024;   // histograms up to this length are read from shared memory
+constexpr int KLD_QLOG = 128;              // bins whose logarithms a warp keeps; with more (the calibration uses 128 and 8) every
+                                           // element works out its bin's
 
 struct KldWarp {
-  double qlog[128];
+  double qlog[KLD_QLOG];
 };
 
 __global__ void __launch_bounds__(KLD_WARPS * 32)
@@ -459,7 +461,8 @@ kld_kernel(const KldTensor* __restrict__ tab, int BINS, float* __restrict__ kl_a
   }
   const float sum = __shfl_sync(0xffffffffu, chain, 0), tail = __shfl_sync(0xffffffffu, chain, 1);
   double* const qlog = per_warp[warp].qlog;
-  for (int b = lane; b < BINS; b += 32) {
+  const bool kept = BINS <= KLD_QLOG;
+  auto q_log = [&](int b) {
     float sum_bin = 0.f;
     int positive = 0;
     for (int k = 0; k < expand; ++k) {
@@ -468,8 +471,10 @@ kld_kernel(const KldTensor* __restrict__ tab, int BINS, float* __restrict__ kl_a
       positive += h > 0;
     }
     const float q = __fdiv_rn(__fdiv_rn(sum_bin, positive ? (float)positive : 1.f), sum);
-    qlog[b] = log10(__dadd_rn((double)q, 1e-30));
-  }
+    return log10(__dadd_rn((double)q, 1e-30));
+  };
+  if (kept)
+    for (int b = lane; b < BINS; b += 32) qlog[b] = q_log(b);
   __syncwarp();
   const double qlog0 = log10(__dadd_rn(0.0, 1e-30));
   float acc = 0.f;
@@ -479,7 +484,7 @@ kld_kernel(const KldTensor* __restrict__ tab, int BINS, float* __restrict__ kl_a
     const float p = idx < i ? __fdiv_rn(idx == i - 1 ? tail : (float)h, fcount) : 0.f;
     double term = 0.0;
     if (p != 0.f)
-      term = __dmul_rn((double)p, __dsub_rn(log10(__dadd_rn((double)p, 1e-30)), h ? qlog[idx / expand] : qlog0));
+      term = __dmul_rn((double)p, __dsub_rn(log10(__dadd_rn((double)p, 1e-30)), !h ? qlog0 : (kept ? qlog[idx / expand] : q_log(idx / expand))));
     // p == 0: the term is exactly +-0 and leaves the accumulator unchanged
     unsigned live = __ballot_sync(0xffffffffu, p != 0.f);
     if (live == 0xffffffffu) {
@@ -670,7 +675,7 @@ int fold_launch(const int* in, long long n_in, int* out, long long n_out, cudaSt
 
 int kld_launch(const KldTensor* tab_dev, int tensors, int dst_bins, long long max_len, float* thresholds_dev, float* kl_dev, cudaStream_t s) {
   if (tensors == 0) return B200Q_OK;
-  if (dst_bins < 1 || dst_bins > 128 || max_len / dst_bins > 1024)
+  if (dst_bins < 1 || max_len / dst_bins > 1024)
     return set_error(B200Q_ERR_UNSUPPORTED, "kld: more than 1024 candidates (fold the histogram to at most %d bins first)", 1024 * dst_bins);
   const int smem_bins = max_len < KLD_SMEM_BINS ? (int)max_len : KLD_SMEM_BINS;
   const size_t smem = KLD_WARPS * sizeof(KldWarp) + (size_t)smem_bins * 4;
