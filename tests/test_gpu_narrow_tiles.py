@@ -65,3 +65,27 @@ def test_channels_last_conv(n, h, w, oc, qdm):
         L.lib().b200q_conv2d_dev_destroy(C.byref(hd))
         outs.append(y.permute(0, 3, 1, 2) if nhwc else y)
     assert torch.equal(outs[0].contiguous(), outs[1]) and outs[1].float().std() > 10
+
+
+@pytest.mark.parametrize("M,N", [(64, 4096), (128, 12544), (128, 12545), (100, 6145), (129, 6144), (129, 6400), (257, 300)])
+@pytest.mark.parametrize("f16", [False, True])
+def test_a16_prompts(M, N, f16):
+    """The 16-bit products of a 4-bit-weight handle in tiles of every width.  Integer activations and power-of-two scales: every sum
+    is exact in fp32, so the outputs are the reference's rounding bit for bit."""
+    import oracle
+    K, g = 192, 64
+    rng = np.random.default_rng(M + N)
+    q = rng.integers(0, 16, size=(N, K), dtype=np.uint8)
+    wq = (q[:, 0::2] | (q[:, 1::2] << 4)).astype(np.uint8)
+    sc = (2.0**-9 * rng.choice([1.0, 2.0, 4.0], N * K // g)).astype(np.float32)
+    zp = rng.integers(0, 16, size=N * K // g, dtype=np.uint8)
+    x = rng.integers(-3, 4, size=(M, K)).astype(np.float32)
+    bits = (lambda a: a.astype(np.float16).view(np.uint16)) if f16 else (lambda a: (a.view(np.uint32) >> 16).astype(np.uint16))
+    ref = oracle.a16matmul_w4(bits(x), wq, bits(sc), zp, group=g, f16=f16)
+    d = [torch.from_numpy(a).cuda() for a in (bits(x).copy(), wq, bits(sc).copy(), zp)]
+    y, h = torch.zeros((M, N), dtype=torch.uint16, device="cuda"), C.c_void_p()
+    L.check(L.lib().b200q_a16_dev_create_dt(ptr(d[1]), ptr(d[2]), ptr(d[3]), None, N, K, g, L.DT_F16 if f16 else L.DT_BF16, C.byref(h)))
+    L.check(L.lib().b200q_a16_dev_run(h, ptr(d[0]), ptr(y), M, None))
+    L.check(L.lib().b200q_a16_dev_status(h, None))
+    L.lib().b200q_a16_dev_destroy(C.byref(h))
+    assert np.array_equal(y.cpu().numpy(), ref)

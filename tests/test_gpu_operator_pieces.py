@@ -29,7 +29,9 @@ def _matmul(M, K, N, seed, out_dtype=L.DT_I8, signed=True):
 
 
 @pytest.mark.parametrize("M,K,N", [(1, 16, 1), (3, 32, 33), (500, 96, 40), (PIECE // 1024, 1024, 8), (PIECE // 1024 + 1, 1024, 8),
-                                   (5 * (PIECE // 2048) + 7, 2048, 24), (6 * 1024 + 1, 64, 512)])
+                                   (5 * (PIECE // 2048) + 7, 2048, 24), (6 * 1024 + 1, 64, 512),
+                                   # rows off 16 bytes: the pieces start anywhere, the products run on the CUDA cores
+                                   (5 * (PIECE // 777) + 3, 777, 24), (9001, 33, 131), (PIECE // 1001 + 2, 1001, 40)])
 def test_rows_over_pieces(M, K, N):
     op, p, want = _matmul(M, K, N, M)
     op.init(p)
